@@ -31,6 +31,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE
 # says why).
 UNITS = {
     "rk4_f64.cu": ["-fmad=false"],
+    "rk4_f64_grid.cu": ["-fmad=false"],
     "api.cu": [],
     "netcdf3.cpp": [],
     "diag.cu": [],

@@ -149,6 +149,99 @@ void fill_bathy_grid_scalars(mr_bathymetry *h, const float *x, const float *y, s
   d.yspace = static_cast<double>(y[1]) - static_cast<double>(y[0]);
 }
 
+// Smallest float t whose index (t - a0) / sp, as the reference computes it in
+// f32, is >= j: bisection over the ordered floats (the index is
+// non-decreasing in t; +inf satisfies the predicate).
+float f32_axis_threshold(float a0, float sp, float j) {
+  auto value = [](int32_t key) {
+    const int32_t bits = key ^ ((key >> 31) & 0x7fffffff);
+    float t;
+    std::memcpy(&t, &bits, sizeof t);
+    return t;
+  };
+  auto key_of = [](float t) {
+    int32_t bits;
+    std::memcpy(&bits, &t, sizeof bits);
+    return bits ^ ((bits >> 31) & 0x7fffffff);
+  };
+  int64_t lo = key_of(-INFINITY), hi = key_of(INFINITY);
+  while (lo < hi) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    const float idx = (value(static_cast<int32_t>(mid)) - a0) / sp;
+    if (idx >= j)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  return value(static_cast<int32_t>(lo));
+}
+
+// Whether the split form's records cover an axis: at least two points,
+// finite, strictly ascending, edges within 2^-60..2^60.
+bool split_axis_ok(const float *a, size_t n) {
+  if (n < 2 || n > (1u << 23)) return false;
+  for (size_t i = 0; i < n; ++i)
+    if (!std::isfinite(a[i])) return false;
+  for (size_t i = 0; i + 1 < n; ++i) {
+    const float e = a[i + 1] - a[i];
+    if (!(e > 0x1p-60f && e < 0x1p60f)) return false;
+  }
+  return true;
+}
+
+// The axis cells (fields.h) from the smallest coordinate of each cell by the
+// field's index rule, as f32: first[i] for i < n.  inclusive: first[i] itself
+// is in cell i (the bathymetry's f32 rule); otherwise it is the f32 rounding
+// of an f64 threshold, and only floats beyond it are certain.
+std::vector<mr::AxisCell> split_axis_cells(const float *a, size_t n,
+                                           const std::vector<float> &first, bool inclusive) {
+  std::vector<mr::AxisCell> c(n - 1);
+  for (size_t i = 0; i + 1 < n; ++i) {
+    const float from = inclusive ? nextafterf(first[i], -INFINITY) : first[i];
+    c[i].lo = a[i] > from ? a[i] : from;
+    c[i].hi = a[i + 1] < first[i + 1] ? a[i + 1] : first[i + 1];
+    c[i].a1 = a[i];
+    // on the lower axis value: certain by the f32 rule, or decided by the f64
+    // coordinate where the threshold rounds to that value
+    const bool in = inclusive ? first[i] <= a[i] : first[i] == a[i];
+    c[i].edge = in && a[i] < first[i + 1] ? a[i] : NAN;
+  }
+  return c;
+}
+
+// Uploads the axis cells and builds the records; without memory for them the
+// handle works as before (the general kernels).
+template <typename Handle, typename Launch>
+cudaError_t make_split(Handle *h, const float *x, const float *y, size_t nx, size_t ny,
+                       const std::vector<float> &fx, const std::vector<float> &fy,
+                       bool inclusive, float spx, float spy, size_t record, Launch launch) {
+  const auto xc = split_axis_cells(x, nx, fx, inclusive);
+  const auto yc = split_axis_cells(y, ny, fy, inclusive);
+  void *rec = nullptr;
+  if (cudaMalloc(&rec, nx * ny * record) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return cudaSuccess;
+  }
+  h->mem.push_back(rec);
+  mr::SplitGrid g{};
+  cudaError_t e = upload(xc.data(), xc.size(), &h->mem, &g.xc);
+  if (e == cudaSuccess) e = upload(yc.data(), yc.size(), &h->mem, &g.yc);
+  if (e == cudaSuccess) e = launch(h->dev, rec, cudaStreamPerThread);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
+  if (e != cudaSuccess) return e;
+  g.rec = rec;
+  g.nx = static_cast<int>(nx);
+  g.ny = static_cast<int>(ny);
+  g.x0 = x[0];
+  g.inv_x = 1.0f / spx;
+  g.y0 = y[0];
+  g.inv_y = 1.0f / spy;
+  h->dev.split = g;
+  h->x32.assign(x, x + nx);
+  h->y32.assign(y, y + ny);
+  return cudaSuccess;
+}
+
 int make_bathy_grid(size_t nx, size_t ny, const float *x, const float *y, const double *depth,
                     size_t depth_len, mr_bathymetry **out) {
   if (!out) return fail(MR_ERR_INVALID_ARGUMENT, "null output handle pointer");
@@ -187,6 +280,19 @@ int make_bathy_grid(size_t nx, size_t ny, const float *x, const float *y, const 
     return cuda_fail(e, "staging bathymetry grid");
   }
   h->dev.depth_len = depth_len;
+  if (split_axis_ok(x, nx) && split_axis_ok(y, ny) && depth_len >= nx * ny &&
+      nx * ny < (1ull << 31)) {
+    std::vector<float> fx(nx), fy(ny);
+    for (size_t i = 0; i < nx; ++i) fx[i] = f32_axis_threshold(x[0], h->dev.xsp, static_cast<float>(i));
+    for (size_t i = 0; i < ny; ++i) fy[i] = f32_axis_threshold(y[0], h->dev.ysp, static_cast<float>(i));
+    e = make_split(h, x, y, nx, ny, fx, fy, true, h->dev.xsp, h->dev.ysp, 32,
+                   mr::launch_bathy_records);
+    if (e != cudaSuccess) {
+      free_mem(h->mem);
+      delete h;
+      return cuda_fail(e, "building bathymetry records");
+    }
+  }
   *out = h;
   return MR_OK;
 }
@@ -313,6 +419,28 @@ int make_current_grid(size_t nx, size_t ny, const double *x, const double *y, co
     delete h;
     return cuda_fail(e, "staging current grid");
   }
+  if (use_thr && split_axis_ok(x32.data(), nx) && split_axis_ok(y32.data(), ny) &&
+      len >= nx * ny && nx * ny < (1ull << 31)) {
+    // the thresholds of the f64 index rule as f32
+    auto first = [](const std::vector<long long> &thr, size_t n) {
+      std::vector<float> f(n);
+      for (size_t i = 0; i < n; ++i) {
+        const long long bits = mr::order_key_bits(thr[i]);
+        double t;
+        std::memcpy(&t, &bits, sizeof t);
+        f[i] = static_cast<float>(t);
+      }
+      return f;
+    };
+    e = make_split(h, x32.data(), y32.data(), nx, ny, first(xthr, nx), first(ythr, ny), false,
+                   static_cast<float>(d.xsp), static_cast<float>(d.ysp), 80,
+                   mr::launch_current_records);
+    if (e != cudaSuccess) {
+      free_mem(h->mem);
+      delete h;
+      return cuda_fail(e, "building current records");
+    }
+  }
   *out = h;
   return MR_OK;
 }
@@ -331,8 +459,9 @@ int launch(const mr_bathymetry *b, const mr_current *c, size_t n, const double *
   a.traj = traj;
   a.n_rows = n_rows;
   a.status = status;
+  const bool same_axes = !b->x32.empty() && b->x32 == c->x32 && b->y32 == c->y32;
   cudaError_t e = mr::launch_rk4_f64(b->dev, c->dev, a, options & MR_STOP_FRESH,
-                                     (options & MR_MATH_LIBM) == 0, stream);
+                                     (options & MR_MATH_LIBM) == 0, same_axes, stream);
   if (e != cudaSuccess) return cuda_fail(e, "rk4_f64 launch");
   return MR_OK;
 }

@@ -35,8 +35,32 @@ enum CurrentKind : int {
   CURRENT_CONSTANT = 1  // ConstantCurrent (constant_current.rs:50-108)
 };
 
+// One cell of an axis for the split integrator (split_lookup.cuh): a point
+// whose f32 coordinate t satisfies lo < t < hi is in the cell by the
+// reference's index rule and strictly between its two f32 axis values; t =
+// edge is the cell's own lower axis value, in the cell by that rule (for the
+// current: if the f64 coordinate is at or above the cell's threshold); edge
+// is NaN where the lower axis value is not in the cell.
+struct AxisCell { float lo, hi, a1, edge; };
+
+// What the split integrator reads of a gridded field: one AxisCell per cell
+// of each axis and one record per cell, by its south-west node (nx*j + i).
+// Bathymetry, 32 B: the four bilinear coefficients a00, a10, a01, a11
+// (lookup.cuh, CellWeights), dh/dx, dh/dy, m01, m10.  Current, 80 B: the
+// coefficients of u, of v, the four gradients as (high, low) float pairs,
+// m01, m10 and two unused floats.  All null when the grid is outside what the
+// records cover (fewer than two points an axis, axes not ascending and
+// finite, arrays shorter than the grid, 2^31 nodes or more).
+struct SplitGrid {
+  const AxisCell *xc, *yc;
+  const void *rec;         // float4 [nx * ny][2] or [5]
+  int nx, ny;
+  float x0, inv_x, y0, inv_y;  // first guess of the cell (checked against AxisCell)
+};
+
 struct BathyDev {
   int kind;
+  SplitGrid split;
   uint64_t nx, ny;
   const float *x;        // [nx] axis (f32, as the reference stores it)
   const float *y;        // [ny]
@@ -59,6 +83,7 @@ struct BathyDev {
 
 struct CurrentDev {
   int kind;
+  SplitGrid split;
   uint64_t nx, ny;
   const double *x;   // [nx] f64 axes
   const double *y;   // [ny]

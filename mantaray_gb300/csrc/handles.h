@@ -13,6 +13,7 @@ struct mr_bathymetry {
   int device = 0;
   bool one_point_axis = false;  // the reference panics on its first lookup
   std::vector<void *> mem;      // device allocations owned by the handle
+  std::vector<float> x32, y32;  // host copies of the axes as f32 (grids)
 };
 
 struct mr_current {
@@ -20,6 +21,7 @@ struct mr_current {
   int device = 0;
   bool one_point_axis = false;
   std::vector<void *> mem;
+  std::vector<float> x32, y32;  // host copies of the axes as f32 (grids)
 };
 
 namespace mr {

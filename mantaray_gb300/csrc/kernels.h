@@ -24,8 +24,18 @@ struct TraceArgs {
   uint8_t *status;            // [n]
 };
 
+// same_axes: both fields gridded on equal f32 axes.
 cudaError_t launch_rk4_f64(const BathyDev &b, const CurrentDev &c, const TraceArgs &a,
-                           int stop_rule, int identity_math, cudaStream_t stream);
+                           int stop_rule, int identity_math, int same_axes, cudaStream_t stream);
+
+// The split form (rk4_f64_grid.cu): whether it covers the call, its launch,
+// and the per-cell records it reads (nx * ny records of 32 / 80 bytes).
+bool split_covers(const BathyDev &b, const CurrentDev &c, const TraceArgs &a);
+cudaError_t launch_rk4_f64_grid(const BathyDev &b, const CurrentDev &c, const TraceArgs &a,
+                                int stop_rule, int same_axes, unsigned grid, int block,
+                                cudaStream_t stream);
+cudaError_t launch_bathy_records(const BathyDev &b, void *rec, cudaStream_t stream);
+cudaError_t launch_current_records(const CurrentDev &c, void *rec, cudaStream_t stream);
 
 // Batched FP32 form: cell packing of one field (one thread per cell) and the
 // persistent integrator (grid = SMs x blocks_per_sm).

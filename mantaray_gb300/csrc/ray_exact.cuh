@@ -183,4 +183,24 @@ __device__ __forceinline__ bool all_nan4(const double v[4]) {
   return nan_bits(v[0]) && nan_bits(v[1]) && nan_bits(v[2]) && nan_bits(v[3]);
 }
 
+// Row `row` of ray i in traj[5][rows][n] (plane = rows * n).
+__device__ __forceinline__ void store_row(double *traj, uint64_t plane, uint64_t n,
+                                          uint64_t row, uint64_t i, double t,
+                                          const double y[4]) {
+  double *p = traj + row * n + i;
+  p[0] = t;
+  p[plane] = y[0];
+  p[2 * plane] = y[1];
+  p[3 * plane] = y[2];
+  p[4 * plane] = y[3];
+}
+
+__device__ __forceinline__ void store_nan_row(double *traj, uint64_t plane, uint64_t n,
+                                              uint64_t row, uint64_t i) {
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  double *p = traj + row * n + i;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) p[v * plane] = nan;
+}
+
 }  // namespace mr

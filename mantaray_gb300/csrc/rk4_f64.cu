@@ -29,25 +29,6 @@ namespace mr {
 
 namespace {
 
-__device__ __forceinline__ void store_row(double *traj, uint64_t plane, uint64_t n,
-                                          uint64_t row, uint64_t i, double t,
-                                          const double y[4]) {
-  double *p = traj + row * n + i;
-  p[0] = t;
-  p[plane] = y[0];
-  p[2 * plane] = y[1];
-  p[3 * plane] = y[2];
-  p[4 * plane] = y[3];
-}
-
-__device__ __forceinline__ void store_nan_row(double *traj, uint64_t plane, uint64_t n,
-                                              uint64_t row, uint64_t i) {
-  const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  double *p = traj + row * n + i;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) p[v * plane] = nan;
-}
-
 // One RK4 step as four right-hand-side evaluations in a rolled loop (one copy
 // of the inlined right-hand side in the kernel, which keeps it in the
 // instruction cache): stages 0-2 evaluate at y + k h/2, y + k h/2, y + k h
@@ -166,7 +147,7 @@ static void launch_k1(int stop_rule, unsigned grid, int block, const BathyDev &b
 }
 
 cudaError_t launch_rk4_f64(const BathyDev &b, const CurrentDev &c, const TraceArgs &a,
-                           int stop_rule, int identity_math, cudaStream_t stream) {
+                           int stop_rule, int identity_math, int same_axes, cudaStream_t stream) {
   if (a.n == 0) return cudaSuccess;
   // Blocks of 64 rays, or fewer when that leaves SMs without a block: on
   // GB300 an SM issues 2 FP64 lanes per clock, so a small call runs fastest
@@ -178,6 +159,12 @@ cudaError_t launch_rk4_f64(const BathyDev &b, const CurrentDev &c, const TraceAr
   int block = kK1Block;
   while (block > 8 && (a.n + block - 1) / block < static_cast<uint64_t>(sms)) block /= 2;
   const unsigned grid = static_cast<unsigned>((a.n + block - 1) / block);
+  // Gridded bathymetry with the identity arithmetic takes the split form at
+  // every size: 3.1-3.5x as fast from one ray to 65,536 (rk4_f64_grid.cu).
+  // Analytic depths stay here: their lookups have no f32 interpolation, the
+  // FP64 rounding of a step is their only error.
+  if (identity_math && split_covers(b, c, a))
+    return launch_rk4_f64_grid(b, c, a, stop_rule, same_axes, grid, block, stream);
   // The lookup cache shortens the rays' dependent chains (1,024-16,384 rays:
   // 6-18% faster; the 65,536-ray seamount, identity arithmetic: 2.09 ->
   // 2.15 G ray-steps/s, bit-identical) but takes registers (identity 128 a

@@ -14,6 +14,7 @@ use std::process::Command;
 /// builds with FP32 subnormals flushed as well.
 const UNITS: &[(&str, &[&str])] = &[
     ("rk4_f64.cu", &["-fmad=false"]),
+    ("rk4_f64_grid.cu", &["-fmad=false"]),
     ("api.cu", &[]),
     ("netcdf3.cpp", &[]),
     ("diag.cu", &[]),
@@ -57,8 +58,9 @@ fn build_library(root: &Path, out: &Path) -> PathBuf {
             .arg("-o").arg(&obj));
         objects.push(obj);
     }
-    for header in ["batch.h", "batch_handle.h", "bits.h", "fields.h", "handles.h", "k2.cuh",
-                   "kernels.h", "lookup.cuh", "netcdf3.h", "ray_exact.cuh"] {
+    for header in ["batch.h", "batch_handle.h", "bits.h", "exp_table.h", "fields.h", "handles.h",
+                   "k2.cuh", "kernels.h", "lookup.cuh", "netcdf3.h", "ray_exact.cuh", "split.cuh",
+                   "split_lookup.cuh"] {
         println!("cargo:rerun-if-changed={}", csrc.join(header).display());
     }
     println!("cargo:rerun-if-changed={}", include.join("mantaray_gpu.h").display());
