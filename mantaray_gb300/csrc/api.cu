@@ -209,6 +209,16 @@ std::vector<mr::AxisCell> split_axis_cells(const float *a, size_t n,
   return c;
 }
 
+// SplitGrid's uniform: the axis cells follow from fma(i, sp, a0).
+bool split_axis_uniform(const std::vector<mr::AxisCell> &c, float a0, float sp) {
+  for (size_t i = 0; i < c.size(); ++i) {
+    const float v = fmaf(static_cast<float>(i), sp, a0);
+    const float w = fmaf(static_cast<float>(i + 1), sp, a0);
+    if (c[i].lo != v || c[i].hi != w || c[i].a1 != v || c[i].edge != v) return false;
+  }
+  return true;
+}
+
 // Uploads the axis cells and builds the records; without memory for them the
 // handle works as before (the general kernels).
 template <typename Handle, typename Launch>
@@ -236,6 +246,10 @@ cudaError_t make_split(Handle *h, const float *x, const float *y, size_t nx, siz
   g.inv_x = 1.0f / spx;
   g.y0 = y[0];
   g.inv_y = 1.0f / spy;
+  g.sp_x = spx;
+  g.sp_y = spy;
+  g.uniform_x = split_axis_uniform(xc, x[0], spx);
+  g.uniform_y = split_axis_uniform(yc, y[0], spy);
   h->dev.split = g;
   h->x32.assign(x, x + nx);
   h->y32.assign(y, y + ny);

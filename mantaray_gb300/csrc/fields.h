@@ -46,9 +46,9 @@ struct AxisCell { float lo, hi, a1, edge; };
 // What the split integrator reads of a gridded field: one AxisCell per cell
 // of each axis and one record per cell, by its south-west node (nx*j + i).
 // Bathymetry, 32 B: the four bilinear coefficients a00, a10, a01, a11
-// (lookup.cuh, CellWeights), dh/dx, dh/dy, m01, m10.  Current, 80 B: the
-// coefficients of u, of v, the four gradients as (high, low) float pairs,
-// m01, m10 and two unused floats.  All null when the grid is outside what the
+// (lookup.cuh, CellWeights), dh/dx, dh/dy, m01, m10.  Current, 80 B: (u00,
+// v00, u10, v10), (u01, v01, u11, v11), the gradients as float pairs (du/dx,
+// du/dy: high, high, low, low; then v's), m01, m10 and two unused floats.  All null when the grid is outside what the
 // records cover (fewer than two points an axis, axes not ascending and
 // finite, arrays shorter than the grid, 2^31 nodes or more).
 struct SplitGrid {
@@ -56,6 +56,10 @@ struct SplitGrid {
   const void *rec;         // float4 [nx * ny][2] or [5]
   int nx, ny;
   float x0, inv_x, y0, inv_y;  // first guess of the cell (checked against AxisCell)
+  // uniform: every AxisCell of the axis is {v(i), v(i + 1), v(i), v(i)} with
+  // v(i) = fma(i, sp, a0), so it is computed instead of loaded
+  float sp_x, sp_y;
+  int uniform_x, uniform_y;
 };
 
 struct BathyDev {

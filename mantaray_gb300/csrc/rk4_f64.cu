@@ -160,7 +160,7 @@ cudaError_t launch_rk4_f64(const BathyDev &b, const CurrentDev &c, const TraceAr
   while (block > 8 && (a.n + block - 1) / block < static_cast<uint64_t>(sms)) block /= 2;
   const unsigned grid = static_cast<unsigned>((a.n + block - 1) / block);
   // Gridded bathymetry with the identity arithmetic takes the split form at
-  // every size: 3.1-3.5x as fast from one ray to 65,536 (rk4_f64_grid.cu).
+  // every size: 4.1-4.8x as fast from one ray to 65,536 (rk4_f64_grid.cu).
   // Analytic depths stay here: their lookups have no f32 interpolation, the
   // FP64 rounding of a step is their only error.
   if (identity_math && split_covers(b, c, a))

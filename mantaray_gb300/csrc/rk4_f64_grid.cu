@@ -3,19 +3,29 @@
 // anchor a step (split.cuh) and its lookups from per-cell records
 // (split_lookup.cuh).  One ray per thread, the rows of rk4_f64.cu.
 //
-// A step in the domain of split_ok runs about 40 (deep water) to 70 FP64
-// operations instead of 190 to 370.  A step that leaves that domain at any
-// stage (a ray past the grid, dry or NaN nodes, k = 0) is taken again with
-// the FP64 form of ray_exact.cuh, which also decides how the ray stops: NaN
-// rows and row counts are that form's.  Every ray's arithmetic depends on
-// its own state only, so a ray's rows are the same in every call.
+// A step in the domain of split_ok runs 23 (deep water) to 45 FP64
+// operations instead of 190 to 370, and 1,570 to 2,200 instructions instead
+// of 4,060 to 5,080.  A step that leaves that domain at any stage (a ray past
+// the grid, dry or NaN nodes, k = 0) is taken again with the FP64 form of
+// ray_exact.cuh, which also decides how the ray stops: NaN rows and row
+// counts are that form's.  Every ray's arithmetic depends on its own state
+// only, so a ray's rows are the same in every call.
+//
+// Bounds: few rays, the dependent chain of a step (FP32 4.3 cycles a link,
+// FP64 64); many rays, the chain and the issue slots (55% busy, the FP64 pipe
+// 51%, at the 13.5 warps an SM that 65,536 rays give).  128 registers: 7
+// blocks of 64 per SM are what 65,536 rays need to be resident at once; with
+// 156 they ran in two waves, 24 ms against 15 for the same code.
 //
 // Measured against the FP64 form (GB300, full trajectories): the seamount,
-// 65,536 rays x 2,000 steps, 59.7 -> 17.0 ms (2.19 -> 7.7 G ray-steps/s);
-// the planar beach, 1,024 rays x 2,000 steps, 41.3 -> 13.0 ms; one ray x 200
-// steps 3.78 -> 1.20 ms.  Against the model in 64 bits the trajectories'
-// error is unchanged (seamount 3.7e-12, beach 3.8e-10: the lookups' f32
-// interpolation), and the two forms' rows differ by 4e-16 to 1.4e-15.
+// 65,536 rays x 2,000 steps, 59.7 -> 12.4 ms (2.19 -> 10.5 G ray-steps/s);
+// the planar beach, 1,024 rays x 2,000 steps, 41.3 -> 9.4 ms; one ray x 200
+// steps 3.77 -> 0.84 ms.  Against the model in 64 bits the trajectories'
+// error is unchanged (seamount 5e-12, beach 4e-10: the lookups' f32
+// interpolation).  Against the same lookups with the rest in 80-bit
+// arithmetic (800 rays x 500 to 1,000 steps over a shoal and a jet) the
+// positions' median error is 1.03-1.04 times the FP64 form's, 3.2e-11 and
+// 4.6e-11 m, of which the rounding of the FP64 state is nearly all.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -30,7 +40,7 @@ namespace {
 
 struct StepConst {
   double dt, half, sixth;
-  F2 dt2, half2;  // dt and dt/2 as pairs
+  F2 dt2, half2, sixth2;  // the same as pairs
 };
 
 // The FP64 form's step from y (ray_exact.cuh, rk4_f64.cu).  Returns whether
@@ -70,55 +80,81 @@ __device__ __noinline__ bool fp64_stopped(const BathyDev &b, const CurrentDev &c
   return all_nan4(k);
 }
 
+// f32 coordinates of the position (h + m + r) + inc: RN of the sum, as the
+// FP64 form rounds its stage positions.  The remainder R carries 24 bits; a
+// sum whose rounding they do not decide (1 in 10^6) returns false.
+__device__ __forceinline__ bool stage_point(const V &h, const V &m, const V &r, const V2 &inc,
+                                            V *out) {
+  const V2 s = two_sum(inc.h, m);
+  const V2 t = two_sum(h, s.h);
+  const V R = vadd(t.l, vadd(s.l, vadd(inc.l, r)));
+  const V a = vfma(R, both(1.0f + 0x1p-20f), t.h), b = vfma(R, both(1.0f - 0x1p-20f), t.h);
+  *out = a;
+  return a.x == b.x && a.y == b.y;
+}
+
 // One step in pairs; false (y unchanged) when any stage is outside split_ok.
+// The last three stages run in a rolled loop: two copies of the lookups and
+// of the right-hand side, which the instruction cache holds (the loop
+// unrolled is 1.6x slower).
 template <int CUR>
 __device__ __forceinline__ bool split_step(const BathyDev &b, const CurrentDev &c,
                                            const StepConst &h, SplitCell<CUR> &C, double y[4]) {
-  Sample s;
-  if (!split_sample<CUR>(b, c, y[0], y[1], C, s)) return false;
+  V xh, xm, xr;
+  split3(y[0], &xh.x, &xm.x, &xr.x);
+  split3(y[1], &xh.y, &xm.y, &xr.y);
   const F2 kx = to_pair(y[2]), ky = to_pair(y[3]);
-  F2 k2 = add_pos(sqr(kx), sqr(ky));
-  bool ok = split_ok(s, k2.h);
-  if (!ok) return false;
-  F2 d1[4], d[4];
-  Anchor an;
-  split_rhs<true>(s, kx, ky, k2, d1, &an);
-  const double w = anchor_speed(an, y[2], y[3], s.h);
-  const double ax = fma(w, y[2], CUR == SPLIT_CONSTANT ? c.cu : to_double(s.u));
-  const double ay = fma(w, y[3], CUR == SPLIT_CONSTANT ? c.cv : to_double(s.v));
-  F2 ex = F2{0.0f, 0.0f}, ey = ex;        // the stage's d - d1 in x and y
-  F2 sx = ex, sy = ex;                    // their weighted sums
-  F2 skx = d1[2], sky = d1[3];
-  d[2] = d1[2];
-  d[3] = d1[3];
+  const V2 k = V2{V{kx.h, ky.h}, V{kx.l, ky.l}};
+  Wave wv = wave_of(k);
+  Sample s;
+  if (!split_sample<CUR>(b, c, d2f(y[0]), d2f(y[1]), [&](double *px, double *py) {
+        *px = y[0];
+        *py = y[1];
+      }, C, s))
+    return false;
+  bool ok = split_ok(s, wv.k2.h);
+  V2 d1, d, dk;
+  double w;
+  split_rhs<true>(s, wv, &d1, &dk, y[2], y[3], &w);
+  // gridded currents are f32 values: their low halves are 0
+  const double ax = fma(w, y[2], CUR == SPLIT_CONSTANT ? c.cu : f2d(s.uv.h.x));
+  const double ay = fma(w, y[3], CUR == SPLIT_CONSTANT ? c.cv : f2d(s.uv.h.y));
+  V2 sd = zero2(), sk = dk;               // weighted sums of d - d1 and of dk
+  d = d1;
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {
-    const double hs = st == 2 ? h.dt : h.half;
-    const F2 hs2 = st == 2 ? h.dt2 : h.half2;
-    const double px = fma(hs, to_double(ex), fma(hs, ax, y[0]));
-    const double py = fma(hs, to_double(ey), fma(hs, ay, y[1]));
-    const F2 qx = add(kx, mul(hs2, d[2])), qy = add(ky, mul(hs2, d[3]));
-    if (!split_sample<CUR>(b, c, px, py, C, s)) return false;
-    k2 = add_pos(sqr(qx), sqr(qy));
-    if (!split_ok(s, k2.h)) return false;
-    split_rhs<false>(s, qx, qy, k2, d, nullptr);
-    ex = add(d[0], neg(d1[0]));
-    ey = add(d[1], neg(d1[1]));
+    if (!ok) return false;  // tested where the branches already are
+    const F2 hs = st == 2 ? h.dt2 : h.half2;
+    wv = wave_of(add(k, mul(dk, both(hs))));
+    V t;
+    auto at = [&](double *px, double *py) {
+      const double hd = st == 2 ? h.dt : h.half;
+      *px = fma(hd, to_double(x_of(d)), y[0]);
+      *py = fma(hd, to_double(y_of(d)), y[1]);
+    };
+    if (!stage_point(xh, xm, xr, mul(d, both(hs)), &t)) {
+      double px, py;
+      at(&px, &py);
+      t = V{d2f(px), d2f(py)};
+    }
+    if (!split_sample<CUR>(b, c, t.x, t.y, at, C, s)) return false;
+    ok = split_ok(s, wv.k2.h);
+    split_rhs<false>(s, wv, &d, &dk, 0.0, 0.0, nullptr);
     const float wt = st == 2 ? 1.0f : 2.0f;
-    sx = add(sx, F2{wt * ex.h, wt * ex.l});
-    sy = add(sy, F2{wt * ey.h, wt * ey.l});
-    skx = add(skx, F2{wt * d[2].h, wt * d[2].l});
-    sky = add(sky, F2{wt * d[3].h, wt * d[3].l});
+    sd = add(sd, scale(wt, sub(d, d1)));
+    sk = add(sk, scale(wt, dk));
   }
-  y[0] += fma(h.sixth, to_double(sx), h.dt * ax);
-  y[1] += fma(h.sixth, to_double(sy), h.dt * ay);
-  y[2] = fma(h.sixth, to_double(skx), y[2]);
-  y[3] = fma(h.sixth, to_double(sky), y[3]);
+  if (!ok) return false;
+  const V2 e = mul(sd, both(h.sixth2));
+  y[0] += fma(h.dt, ax, f2d_zero(e.h.x)) + f2d_zero(e.l.x);
+  y[1] += fma(h.dt, ay, f2d_zero(e.h.y)) + f2d_zero(e.l.y);
+  y[2] = fma(h.sixth, to_double(x_of(sk)), y[2]);
+  y[3] = fma(h.sixth, to_double(y_of(sk)), y[3]);
   return true;
 }
 
 template <int STOP_RULE, int CUR>
-__global__ void __launch_bounds__(kK1Block)
+__global__ void __launch_bounds__(kK1Block, 8)
     rk4_f64_grid_kernel(const __grid_constant__ BathyDev b, const __grid_constant__ CurrentDev c,
                         const __grid_constant__ TraceArgs a, const StepConst h) {
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -218,15 +254,15 @@ __global__ void build_current_records(CurrentDev c, float4 *rec) {
                   small_gradient(g[3]);
   float4 *r = rec + 5 * k;
   if (!ok) {
-    r[0] = r[1] = make_float4(f32_nan(), 0.0f, 0.0f, 0.0f);
+    r[0] = r[1] = make_float4(f32_nan(), f32_nan(), 0.0f, 0.0f);
     r[2] = r[3] = r[4] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     return;
   }
-  r[0] = make_float4(W.a00[0], W.a10[0], W.a01[0], W.a11[0]);
-  r[1] = make_float4(W.a00[1], W.a10[1], W.a01[1], W.a11[1]);
+  r[0] = make_float4(W.a00[0], W.a00[1], W.a10[0], W.a10[1]);
+  r[1] = make_float4(W.a01[0], W.a01[1], W.a11[0], W.a11[1]);
   const F2 ux = to_pair(g[0]), uy = to_pair(g[1]), vx = to_pair(g[2]), vy = to_pair(g[3]);
-  r[2] = make_float4(ux.h, ux.l, uy.h, uy.l);
-  r[3] = make_float4(vx.h, vx.l, vy.h, vy.l);
+  r[2] = make_float4(ux.h, uy.h, ux.l, uy.l);
+  r[3] = make_float4(vx.h, vy.h, vx.l, vy.l);
   r[4] = make_float4(W.m01, W.m10, 0.0f, 0.0f);
 }
 
@@ -279,6 +315,7 @@ cudaError_t launch_rk4_f64_grid(const BathyDev &b, const CurrentDev &c, const Tr
   h.sixth = a.dt / 6.0;
   h.dt2 = host_pair(h.dt);
   h.half2 = host_pair(h.half);
+  h.sixth2 = host_pair(h.sixth);
   const int cur = c.kind != CURRENT_GRID ? SPLIT_CONSTANT : same_axes ? SPLIT_SAME : SPLIT_GRID;
   if (stop_rule == 1)
     launch_cur<1>(cur, grid, block, b, c, a, h, stream);

@@ -22,16 +22,16 @@ int main() {
     // depths 0.01 m to 8 km, |k| 1e-3 to 3 rad/m (kh from 1e-5 to 2e4)
     Sample s = {};
     s.h = expf(static_cast<float>(log(0.01) + uniform() * log(8000 / 0.01)));
-    s.gx = 0.125f;
+    s.g.x = 0.125f;
     const double k = exp(log(0.001) + uniform() * log(3000.0)), th = 6.283185307179586 * uniform();
     const double kx = k * cos(th), ky = k * sin(th);
     const F2 px = to_pair(kx), py = to_pair(ky);
-    const F2 k2 = add_pos(sqr(px), sqr(py));
-    if (!split_ok(s, k2.h)) continue;
-    F2 d[4];
-    Anchor an;
-    split_rhs<true>(s, px, py, k2, d, &an);
-    const double w = anchor_speed(an, kx, ky, s.h);
+    const V2 kv = {{px.h, py.h}, {px.l, py.l}};
+    const Wave wave = wave_of(kv);
+    if (!split_ok(s, wave.k2.h)) continue;
+    V2 d, dk;
+    double w;
+    split_rhs<true>(s, wave, &d, &dk, kx, ky, &w);
     const Q g = 9.8, kk = sqrtl(static_cast<Q>(kx) * kx + static_cast<Q>(ky) * ky);
     const Q a = kk * s.h, q = expl(-2 * a), m = -expm1l(-2 * a);
     const Q rho = 1 / sqrtl(kk * m * (1 + q));
@@ -41,13 +41,14 @@ int main() {
     worst_anchor = fmax(worst_anchor, static_cast<double>(fabsl(w / ref - 1)) / 0x1p-49);
     // pairs: some 20 operations of up to 2^-46 each
     const bool xb = fabs(kx) > fabs(ky);
-    const Q dv = static_cast<Q>(xb ? d[0].h : d[1].h) + (xb ? d[0].l : d[1].l);
+    const F2 dp = xb ? x_of(d) : y_of(d), df = x_of(dk);
+    const Q dv = static_cast<Q>(dp.h) + dp.l;
     worst_pair = fmax(worst_pair, static_cast<double>(fabsl(dv / (ref * (xb ? kx : ky)) - 1)) / 0x1p-42);
     // f carries exp(-2a), whose relative error grows with a
     if (a < 22) {
-      const Q fv = (static_cast<Q>(d[2].h) + d[2].l) / 0.125L;
+      const Q fv = (static_cast<Q>(df.h) + df.l) / 0.125L;
       worst_f = fmax(worst_f, static_cast<double>(fabsl(fv / f - 1) / (1 + a)) / 0x1p-42);
-    } else if (d[2].h != 0.0f) {
+    } else if (df.h != 0.0f) {
       worst_f = 2;
     }
     ++checked;
