@@ -327,6 +327,34 @@ MR_SPLIT void split_exp(F2 x, int *n_out, F2 *q, F2 *m) {
   *n_out = n;
 }
 
+// exp(-2a) = q and m = 1 - q in FP64, n as split_exp finds it (8 FP64
+// operations, the table as there).
+MR_SPLIT void anchor_exp(double a, int n, double *q, double *m) {
+  // r/2 = -a + (n/2) ln2/256, the halves exact
+  const double nh = f2d_zero(0.5f * static_cast<float>(n));
+  const double rh = fma(nh, 0x1.cf79abc9e3b3ap-48, fma(nh, 0x1.62e42fefap-9, -a));
+  // p = e^r - 1 = r + 2 (r/2)^2 + r^3/6 + ..., the tail in FP32 (r^3/6 is
+  // below 5e-10)
+  const float rf = 2.0f * d2f(rh);
+  const float tail = rf * rf * rf * fma32(rf, fma32(rf, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f);
+  const double rr = rh + rh;
+  const double p = fma(rr, rh, rr) + f2d(tail);
+#if defined(__CUDA_ARCH__)
+  const double2 tu = __ldg(reinterpret_cast<const double2 *>(kExp64) + (n & 255));
+  double T = tu.x, U = tu.y;
+#else
+  double T = kExp64[n & 255].t, U = kExp64[n & 255].u;
+#endif
+  if (n >= 256) {
+    const uint64_t tb = bits_of(T);
+    T = double_of(static_cast<uint32_t>(tb >> 32) - (static_cast<uint32_t>(n >> 8) << 20),
+                  static_cast<uint32_t>(tb));
+    U = 1.0 - T;
+  }
+  *m = fma(-T, p, U);
+  *q = fma(T, p, T);
+}
+
 // A wavenumber with its square, inverse and magnitude.  Apart from split_rhs
 // so that a stage can compute them beside its position, before its lookup.
 struct Wave {
@@ -398,30 +426,8 @@ MR_SPLIT void split_rhs(const Sample &s, const Wave &wv, V2 *d, V2 *dk, double k
       const double kd = fma(k0, ek, k0);
       const double rkd = fma(rk0, ek, rk0);
       const double ad = kd * f2d_normal(s.h);
-      // r/2 = -a + (n/2) ln2/256, the halves exact
-      const double nh = f2d_zero(0.5f * static_cast<float>(n));
-      const double rh = fma(nh, 0x1.cf79abc9e3b3ap-48, fma(nh, 0x1.62e42fefap-9, -ad));
-      // p = e^r - 1 = r + 2 (r/2)^2 + r^3/6 + ..., the tail in FP32 (r^3/6 is
-      // below 5e-10)
-      const float rf = 2.0f * d2f(rh);
-      const float tail =
-          rf * rf * rf * fma32(rf, fma32(rf, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f);
-      const double rr = rh + rh;
-      const double p = fma(rr, rh, rr) + f2d(tail);
-#if defined(__CUDA_ARCH__)
-      const double2 tu = __ldg(reinterpret_cast<const double2 *>(kExp64) + (n & 255));
-      double T = tu.x, U = tu.y;
-#else
-      double T = kExp64[n & 255].t, U = kExp64[n & 255].u;
-#endif
-      if (n >= 256) {
-        const uint64_t tb = bits_of(T);
-        T = double_of(static_cast<uint32_t>(tb >> 32) - (static_cast<uint32_t>(n >> 8) << 20),
-                      static_cast<uint32_t>(tb));
-        U = 1.0 - T;
-      }
-      const double md = fma(-T, p, U);
-      const double qd = fma(T, p, T);
+      double qd, md;
+      anchor_exp(ad, n, &qd, &md);
       const double q1d = 1.0 + qd;
       const double z0 = f2d_normal(z.h) + f2d_normal(z.l);
       const double zd = fma(z0, fma(-q1d, z0, 1.0), z0);
