@@ -282,7 +282,7 @@ int fill_args(mr_batch *b, size_t n, size_t n_stride, const uint8_t *ray_scenari
   }
   a->scen = b->scen;
   a->scen0 = b->host_scen[0];
-  a->all_same_grid = all_same_grid(b);
+  a->mode = batch_mode(b);
   a->n_scenarios = b->n_scenarios;
   a->ray_scenario = ray_scenario;
   a->n = static_cast<int64_t>(n);
@@ -540,7 +540,7 @@ int mr_batch_graph_create(mr_batch *b, size_t n_max, const uint8_t *ray_scenario
   // the integrator build for this shape, chosen (an occupancy query) before
   // the capture begins
   const void *k2 = mr::rk4_f32_function(cfg->rays_per_lane, cfg->block, cfg->blocks_per_sm,
-                                        b->n_scenarios, all_same_grid(b), cfg->staging,
+                                        batch_mode(b), cfg->staging,
                                         gr->sweep);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {

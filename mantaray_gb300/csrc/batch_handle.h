@@ -49,12 +49,41 @@ struct mr_batch {
   bool has_tmaps = false;
 };
 
+// 1 when an axis of some scenario needs the integrator's wide build.
+inline int wide_axes(const mr_batch *b) {
+  for (const mr::ScenarioDev &s : b->host_scen)
+    for (const mr::PackedGrid *g : {&s.bathy, &s.current})
+      if (g->nx > mr::kNarrowAxis || g->ny > mr::kNarrowAxis) return 1;
+  return 0;
+}
+
 // 1 when every scenario's current is gridded on its bathymetry's grid (the
 // batched kernel then takes one cell lookup for both fields).
 inline int all_same_grid(const mr_batch *b) {
   for (const auto &sc : b->host_scen)
     if (!sc.same_grid) return 0;
   return 1;
+}
+
+// 1 when, besides, every scenario's grid has scenario 0's axes.
+inline int same_geometry(const mr_batch *b) {
+  if (!all_same_grid(b)) return 0;
+  const mr::PackedGrid &g = b->host_scen[0].bathy;
+  for (const auto &sc : b->host_scen) {
+    const mr::PackedGrid &h = sc.bathy;
+    if (h.nx != g.nx || h.ny != g.ny || h.x0 != g.x0 || h.y0 != g.y0 || h.sp_x != g.sp_x ||
+        h.sp_y != g.sp_y || h.inv_sp_x != g.inv_sp_x || h.inv_sp_y != g.inv_sp_y ||
+        h.inv_sp_xd != g.inv_sp_xd || h.inv_sp_yd != g.inv_sp_yd)
+      return 0;
+  }
+  return 1;
+}
+
+// The batched kernel's mode for a batch (k2.cuh).
+inline int batch_mode(const mr_batch *b) {
+  if (wide_axes(b)) return 4;
+  if (b->n_scenarios == 1) return all_same_grid(b) ? 2 : 1;
+  return same_geometry(b) ? 5 : all_same_grid(b) ? 3 : 0;
 }
 
 struct mr_batch_config;

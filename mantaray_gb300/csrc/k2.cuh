@@ -1,7 +1,8 @@
 // k2.cuh -- the batched FP32 integrator's device code (K2), included by the
 // two translation units that instantiate its kernels: rk4_f32.cu (the
-// scenario-table builds: MODE 0, and MODE 3 when every scenario's current is
-// gridded on its bathymetry's grid) and rk4_f32_one.cu (the single-scenario
+// scenario-table builds: MODE 0; MODE 3 when every scenario's current is
+// gridded on its bathymetry's grid, MODE 5 when besides every scenario has the
+// first one's axes; MODE 4 for very long axes) and rk4_f32_one.cu (the single-scenario
 // builds, compiled with FP32 subnormals flushed: MODE 1, and MODE 2 when the
 // current is gridded on the bathymetry's grid).  The design notes are at the
 // top of rk4_f32.cu.
@@ -12,6 +13,7 @@
 #include <stdint.h>
 
 #include "batch.h"
+#include "packed.cuh"
 
 namespace mr {
 
@@ -19,6 +21,7 @@ namespace {
 
 // ------------------------------------------------------------------ K2 --
 
+constexpr int kCappedRegs = 64;  // of the capped builds (below)
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kGf = 9.8f;
 
@@ -67,66 +70,87 @@ __device__ __forceinline__ void one_minus_exp(float x, float &m, float &q) {
   }
 }
 
-// Position of a lane on one grid: the cell of its origin (integral floats:
-// exact, grids have fewer than 2^24 points per axis) plus the origin's
+// Position of a lane on one grid: the cell of its origin plus the origin's
 // fractional cell offset.
 struct GridPos {
-  float fi0, fj0;
-  float f0, g0;
+  int i, j;  // cell column and row
+  V f0;      // fractions
 };
 
 __device__ __forceinline__ GridPos grid_pos(const PackedGrid &g, double ox, double oy) {
   GridPos p;
   const double ux = (ox - g.x0) * g.inv_sp_xd, uy = (oy - g.y0) * g.inv_sp_yd;
   const double fx = floor(ux), fy = floor(uy);
-  // clamp far-away origins (+-1e9 is exact in FP32); such a lane fails the
-  // in-range test of its first lookup
-  p.fi0 = static_cast<float>(fmin(fmax(fx, -1.0e9), 1.0e9));
-  p.fj0 = static_cast<float>(fmin(fmax(fy, -1.0e9), 1.0e9));
-  p.f0 = static_cast<float>(ux - fx);
-  p.g0 = static_cast<float>(uy - fy);
-  if (!(ux == ux) || !(uy == uy)) { p.fi0 = -2.0e9f; p.f0 = 0.0f; }
+  // clamp far-away origins; such a lane fails the in-range test of its first
+  // lookup
+  p.i = static_cast<int>(fmin(fmax(fx, -1.0e9), 1.0e9));
+  p.j = static_cast<int>(fmin(fmax(fy, -1.0e9), 1.0e9));
+  p.f0.x = static_cast<float>(ux - fx);
+  p.f0.y = static_cast<float>(uy - fy);
+  if (!(ux == ux) || !(uy == uy)) { p.i = -1000000000; p.f0.x = 0.0f; }
   return p;
 }
 
-// Cell index and in-cell fractions at offset (px, py) from the origin; false
+// Cell index and in-cell fractions f at offset `at` from the origin; false
 // when outside the grid's cells (or at a NaN position), and the index is then
-// meaningless.  The cell's coordinates are integral floats (exact sums),
-// tested against the grid's bounds.  Cells are indexed in 32 bits (the
-// batch refuses grids of 2^31 cells or more).
-// ix, iy: the cell's column and row (meaningful when inside).
-__device__ __forceinline__ bool locate(const PackedGrid &g, const GridPos &p, float px, float py,
-                                       int *cell, float *fx, float *fy, int *ix, int *iy) {
-  const float ux = fmaf(px, g.inv_sp_x, p.f0);
-  const float uy = fmaf(py, g.inv_sp_y, p.g0);
-  const float flx = floorf(ux), fly = floorf(uy);
-  const float cx = p.fi0 + flx, cy = p.fj0 + fly;
-  // saturating conversions and unsigned arithmetic: defined for any position
-  *ix = __float2int_rz(cx);
-  *iy = __float2int_rz(cy);
+// meaningless.  Cells are indexed in 32 bits (the batch refuses grids of 2^31
+// cells or more).  ix, iy: the cell's column and row (meaningful when inside).
+//
+// floor(u) comes from one addition rounded down: t = u + 1.5 2^23 is the
+// integer floor(u) + 1.5 2^23 for |u| < 2^22, whose bits less those of
+// 1.5 2^23 are floor(u).  No conversion: a stage's two roundings and two
+// float-to-int conversions took 16 of a step's 24 special-function slots
+// (one per 2 clocks and warp) and two of their latencies in a row.  For other u
+// (and NaN) the bits differ from those of 1.5 2^23 by at least 2^22 either
+// way, so the cell lies outside any axis of up to 2^22 points, as the true
+// one does; WIDE (longer axes) converts.
+constexpr float kFloorMagic = 12582912.0f;  // 1.5 2^23
+template <bool WIDE>
+__device__ __forceinline__ bool locate(const PackedGrid &g, const GridPos &p, V at, int *cell,
+                                       V *f, int *ix, int *iy) {
+  const V u = vfma(at, V{g.inv_sp_x, g.inv_sp_y}, p.f0);
+  V fl;
+  if (WIDE) {
+    // integral floats (exact sums: fewer than 2^24 points per axis) and
+    // saturating conversions: defined for any position
+    fl = V{floorf(u.x), floorf(u.y)};
+    *ix = __float2int_rz(static_cast<float>(p.i) + fl.x);
+    *iy = __float2int_rz(static_cast<float>(p.j) + fl.y);
+  } else {
+    const V t = vadd_down(u, both(kFloorMagic));
+    fl = vsub(t, both(kFloorMagic));
+    // unsigned: wraps
+    *ix = static_cast<int>(static_cast<unsigned>(p.i) +
+                           (__float_as_uint(t.x) - __float_as_uint(kFloorMagic)));
+    *iy = static_cast<int>(static_cast<unsigned>(p.j) +
+                           (__float_as_uint(t.y) - __float_as_uint(kFloorMagic)));
+  }
   *cell = static_cast<int>(static_cast<unsigned>(*iy) * static_cast<unsigned>(g.nx - 1) +
                            static_cast<unsigned>(*ix));
-  *fx = ux - flx;
-  *fy = uy - fly;
-  // cx, cy are integral: for finite ones the unsigned test of their
-  // (saturated) conversions is the bounds test 0 <= cx <= nx - 2.  A NaN
-  // position converts to cell (0, 0) and passes it, but its fractions and
-  // so its depth are NaN: the stage fails all the same, with the same
-  // status (out of domain), and cell 0 is a valid load.
+  *f = vsub(u, fl);
+  // A NaN position fails here (WIDE: converts to cell 0, a valid load, and
+  // fails by its NaN depth, with the same status: out of domain).
   return static_cast<unsigned>(*ix) <= static_cast<unsigned>(g.nx - 2) &&
          static_cast<unsigned>(*iy) <= static_cast<unsigned>(g.ny - 2);
 }
 
-__device__ __forceinline__ bool locate(const PackedGrid &g, const GridPos &p, float px, float py,
-                                       int *cell, float *fx, float *fy) {
+template <bool WIDE>
+__device__ __forceinline__ bool locate(const PackedGrid &g, const GridPos &p, V at, int *cell,
+                                       V *f) {
   int ix, iy;
-  return locate(g, p, px, py, cell, fx, fy, &ix, &iy);
+  return locate<WIDE>(g, p, at, cell, f, &ix, &iy);
 }
 
 // c = the cell's bilinear coefficients (batch.h): c.x + c.y fx + c.z fy +
 // c.w fx fy in three FMAs.
-__device__ __forceinline__ float bilin(const float4 &c, float fx, float fy) {
-  return fmaf(fy, fmaf(fx, c.w, c.z), fmaf(fx, c.y, c.x));
+__device__ __forceinline__ float bilin(const float4 &c, V f) {
+  return fmaf(f.y, fmaf(f.x, c.w, c.z), fmaf(f.x, c.y, c.x));
+}
+// The same for u and v at once: a = (u's c.x, v's, u's c.y, v's), b = (u's
+// c.z, v's, u's c.w, v's).
+__device__ __forceinline__ V bilin2(const float4 &a, const float4 &b, V f) {
+  const V fx = both(f.x), fy = both(f.y);
+  return vfma(fy, vfma(fx, V{b.z, b.w}, V{b.x, b.y}), vfma(fx, V{a.z, a.w}, V{a.x, a.y}));
 }
 
 // The cell records a lane read last, kept in registers: a ray stays in one
@@ -136,7 +160,7 @@ struct CellCache {
   int bkey, ckey;         // cell indices held, -1: none
   float4 b0;              // depth's bilinear coefficients
   float bx, by;           // dh/dx, dh/dy
-  float4 c0, c1, c2;      // u's and v's coefficients, the current's gradients
+  float4 c0, c1, c2;      // (u, v) coefficients (bilin2), the current's gradients
 };
 
 // The cell a lane's ray is heading into (the ahead build): its records are
@@ -153,8 +177,8 @@ struct RayLane {
   int scen;
   double ox, oy;    // FP64 origin
   GridPos pb, pc;   // origin on the bathymetry and current grids
-  float px, py, kx, ky;      // offsets and wavenumber
-  float cpx, cpy, ckx, cky;  // Kahan compensations
+  V p, k;           // offsets and wavenumber
+  V cp, ck;         // Kahan compensations
   int32_t step;       // steps taken (max_steps < 2^31)
   int32_t saved;
   int32_t to_save;    // steps until the next decimated row (no 64-bit modulo per step)
@@ -172,9 +196,8 @@ struct RayLane {
 //   c_g = (g/2) (tanh a + a / cosh^2 a) / sqrt(g k tanh a),
 //   dk/dt from the depth = -(k/2) sqrt(g k tanh a) / (sinh a cosh a) grad h;
 // beyond a = 23 (deep water) c_g = (g/2) / sqrt(g k) and no refraction.
-__device__ __forceinline__ void ray_equations(float h, float u, float v, float dudx, float dudy,
-                                              float dvdx, float dvdy, float bx, float by,
-                                              float kx, float ky, float k2, float d[4]) {
+__device__ __forceinline__ void ray_equations(float h, V uv, V du, V dv, V grad, V kv, float k2,
+                                              V *dp, V *dk) {
   const float rk = rsqrt_approx(k2);
   const float k = k2 * rk;
   const float kh = k * h;
@@ -197,10 +220,20 @@ __device__ __forceinline__ void ray_equations(float h, float u, float v, float d
     f = (-0.5f * k) * ((q4 * inv_d) * (gkt * rs));
   }
   const float cgk = cg * rk;            // c_g / k: c_g cos(theta) = cgk kx
-  d[0] = fmaf(cgk, kx, u);
-  d[1] = fmaf(cgk, ky, v);
-  d[2] = fmaf(-ky, dvdx, fmaf(-kx, dudx, f * bx));
-  d[3] = fmaf(-ky, dvdy, fmaf(-kx, dudy, f * by));
+  *dp = vfma(both(cgk), kv, uv);
+  *dk = vfma(both(-kv.y), dv, vfma(both(-kv.x), du, vmul(both(f), grad)));
+}
+
+// A lane's scenario: from the kernel's parameters in the single-scenario
+// builds (MODE 1, 2) and, for all but its records, where every scenario has
+// the same geometry (MODE 5); else from the device table (MODE 0, 3, 4).
+template <int MODE>
+__device__ __forceinline__ const ScenarioDev &scenario(const BatchArgs &a, int s) {
+  return (MODE == 1 || MODE == 2 || MODE == 5) ? a.scen0 : a.scen[s];
+}
+template <int MODE>
+__device__ __forceinline__ const ScenarioDev &cells_of(const BatchArgs &a, int s) {
+  return (MODE == 1 || MODE == 2) ? a.scen0 : a.scen[s];
 }
 
 // The records of bathymetry cell cb, unless the lane holds them.
@@ -225,7 +258,7 @@ __device__ __forceinline__ void load_current_cell(const ScenarioDev &s, CellCach
 }
 
 // The records of cell cb of both fields when the current is gridded on the
-// bathymetry's grid (modes 2 and 3), unless the lane holds them.
+// bathymetry's grid (modes 2, 3 and 5), unless the lane holds them.
 __device__ __forceinline__ void load_same_grid_cell(const ScenarioDev &s, CellCache &C, int cb) {
   if (cb != C.bkey) {
     C.b0 = __ldg(s.bathy.cells + static_cast<int64_t>(cb) * 2);
@@ -277,21 +310,22 @@ __device__ __forceinline__ void load_same_grid_cell_ahead(const ScenarioDev &s, 
 }
 
 // The ahead build's prediction, once a step after the first stage: the
-// neighbour cell the ray leaves its cell into at velocity (vx, vy) (the
+// neighbour cell the ray leaves its cell into at velocity v (the
 // nearer of its x and y exits), whose records are copied into the lane's
 // shared-memory slot now; they are first read when the ray enters that
 // cell, a step or more later, so the copy's latency passes while the lane
 // computes.
 template <int MODE>
-__device__ __forceinline__ void load_ahead(const ScenarioDev &s, RayLane &L, float vx, float vy) {
+__device__ __forceinline__ void load_ahead(const ScenarioDev &s, const ScenarioDev &t, RayLane &L,
+                                           V v) {
   int cb, ix, iy;
-  float fx, fy;
-  if (!locate(s.bathy, L.pb, L.px, L.py, &cb, &fx, &fy, &ix, &iy)) return;
-  const float ux = vx * s.bathy.inv_sp_x, uy = vy * s.bathy.inv_sp_y;  // cells per second
-  const float tx = ux > 0.0f ? (1.0f - fx) * rcp_approx(ux)
-                             : (ux < 0.0f ? fx * rcp_approx(-ux) : 3.0e38f);
-  const float ty = uy > 0.0f ? (1.0f - fy) * rcp_approx(uy)
-                             : (uy < 0.0f ? fy * rcp_approx(-uy) : 3.0e38f);
+  V f;
+  if (!locate<false>(s.bathy, L.pb, L.p, &cb, &f, &ix, &iy)) return;
+  const float ux = v.x * s.bathy.inv_sp_x, uy = v.y * s.bathy.inv_sp_y;  // cells per second
+  const float tx = ux > 0.0f ? (1.0f - f.x) * rcp_approx(ux)
+                             : (ux < 0.0f ? f.x * rcp_approx(-ux) : 3.0e38f);
+  const float ty = uy > 0.0f ? (1.0f - f.y) * rcp_approx(uy)
+                             : (uy < 0.0f ? f.y * rcp_approx(-uy) : 3.0e38f);
   int ni = ix, nj = iy;
   if (tx < ty)
     ni += ux > 0.0f ? 1 : -1;
@@ -306,8 +340,8 @@ __device__ __forceinline__ void load_ahead(const ScenarioDev &s, RayLane &L, flo
   cp_async_wait_all();  // the slot's previous copy has landed before it is overwritten
   const uint32_t slot = static_cast<uint32_t>(__cvta_generic_to_shared(k2_ahead_smem)) +
                         threadIdx.x * 80u;
-  const float4 *b = s.bathy.cells + static_cast<int64_t>(key) * 2;
-  const float4 *c = s.current.cells + static_cast<int64_t>(key) * 3;
+  const float4 *b = t.bathy.cells + static_cast<int64_t>(key) * 2;
+  const float4 *c = t.current.cells + static_cast<int64_t>(key) * 3;
   cp_async16(slot, b);
   cp_async16(slot + 16, b + 1);
   cp_async16(slot + 32, c);
@@ -456,57 +490,56 @@ __device__ __forceinline__ void load_same_grid_cell_tile(const ScenarioDev &s, C
   }
 }
 
-// One right-hand side in FP32 at offset (px, py), wavenumber (kx, ky).
+// One right-hand side in FP32 at offset p, wavenumber k.
 // The fields come from the lane's cell records (loaded when the lane does not
 // hold the cell; a point outside a grid loads nothing and uses the records
 // held, whatever they are, and a NaN point reads cell 0's: its depth is NaN
 // all the same).  With EXACT, returns the stage's BatchStatus: out
 // of domain (outside a grid, or depth NaN: a cell past the depth array), dry
 // (depth <= 0), bad wavenumber (k^2 not in (0, 3e38)), else complete;
-// without, BATCH_COMPLETE or not (the same test, no status code).  d is
-// meaningful only when complete.  Written without early returns so that the
-// four stages of a step run with no branch between them.  MODE 2 and 3: the
+// without, BATCH_COMPLETE or not (the same test, no status code).  dp
+// and dk are meaningful only when complete.  Written without early returns so that the
+// four stages of a step run with no branch between them.  MODE 2, 3 and 5: the
 // current is gridded on the bathymetry's grid, so one cell (one key, one
 // test) serves both fields.  STAGE (MR_STAGING_*): 1 (mode 2), records from
 // the warp's tile when the cell is in it; 2 (modes 2, 3), from the registers
 // loaded ahead when the ray entered the predicted cell.
 template <int MODE, bool EXACT, int STAGE>
-__device__ __forceinline__ int rhs_f32(const ScenarioDev &s, RayLane &L, const WarpTile &W,
-                                       float px, float py, float kx, float ky, float d[4]) {
+__device__ __forceinline__ int rhs_f32(const ScenarioDev &s, const ScenarioDev &t, RayLane &L,
+                                       const WarpTile &W, V p, V k, V *dp, V *dk) {
   CellCache &C = L.cache;
   int cb, ix, iy;
-  float fx, fy;
-  bool inside = locate(s.bathy, L.pb, px, py, &cb, &fx, &fy, &ix, &iy);
-  float u, v, dudx, dudy, dvdx, dvdy;
-  if (MODE == 2 || MODE == 3) {
+  V f;
+  bool inside = locate<MODE == 4>(s.bathy, L.pb, p, &cb, &f, &ix, &iy);
+  V uv, du, dv;
+  if (MODE == 2 || MODE == 3 || MODE == 5) {
     if (STAGE == 1)
       load_same_grid_cell_tile(s, C, W, inside ? cb : C.bkey, ix, iy);
     else if (STAGE == 2)
-      load_same_grid_cell_ahead(s, C, L.next, inside ? cb : C.bkey);
+      load_same_grid_cell_ahead(t, C, L.next, inside ? cb : C.bkey);
     else
-      load_same_grid_cell(s, C, inside ? cb : C.bkey);
-    u = bilin(C.c0, fx, fy);
-    v = bilin(C.c1, fx, fy);
-    dudx = C.c2.x; dudy = C.c2.y; dvdx = C.c2.z; dvdy = C.c2.w;
+      load_same_grid_cell(t, C, inside ? cb : C.bkey);
+    uv = bilin2(C.c0, C.c1, f);
+    du = V{C.c2.x, C.c2.y};
+    dv = V{C.c2.z, C.c2.w};
   } else {
     load_bathy_cell(s, C, inside ? cb : C.bkey);
     if (s.current.kind == 0) {
       int cc = cb;
-      float gx = fx, gy = fy;  // the same cell when the grids coincide (same origin, same arithmetic)
-      if (!s.same_grid) inside &= locate(s.current, L.pc, px, py, &cc, &gx, &gy);
+      V g = f;  // the same cell when the grids coincide (same origin, same arithmetic)
+      if (!s.same_grid) inside &= locate<MODE == 4>(s.current, L.pc, p, &cc, &g);
       load_current_cell(s, C, inside ? cc : C.ckey);
-      u = bilin(C.c0, gx, gy);
-      v = bilin(C.c1, gx, gy);
-      dudx = C.c2.x; dudy = C.c2.y; dvdx = C.c2.z; dvdy = C.c2.w;
+      uv = bilin2(C.c0, C.c1, g);
+      du = V{C.c2.x, C.c2.y};
+      dv = V{C.c2.z, C.c2.w};
     } else {
-      u = s.current.cu;
-      v = s.current.cv;
-      dudx = dudy = dvdx = dvdy = 0.0f;
+      uv = V{s.current.cu, s.current.cv};
+      du = dv = both(0.0f);
     }
   }
-  const float h = bilin(C.b0, fx, fy);
-  const float k2 = fmaf(kx, kx, ky * ky);
-  ray_equations(h, u, v, dudx, dudy, dvdx, dvdy, C.bx, C.by, kx, ky, k2, d);
+  const float h = bilin(C.b0, f);
+  const float k2 = fmaf(k.x, k.x, k.y * k.y);
+  ray_equations(h, uv, du, dv, V{C.bx, C.by}, k, k2, dp, dk);
   const bool wet = h > 0.0f;
   // 0 < k2 < 3e38 on the bit pattern (k2 = kx^2 + ky^2 is +0, positive,
   // +inf or NaN; 3e38 is 0x7f61b1e6): one integer compare
@@ -517,17 +550,19 @@ __device__ __forceinline__ int rhs_f32(const ScenarioDev &s, RayLane &L, const W
   return !wet ? BATCH_DRY : BATCH_BAD_WAVENUMBER;
 }
 
-__device__ __forceinline__ void kahan_add(float &sum, float &comp, float inc) {
-  const float y = inc - comp;
-  const float t = sum + y;
-  comp = (t - sum) - y;
+// sum += w s, compensated, for two components.  The products are scalar: a
+// packed one would be contracted into the difference (packed.cuh).
+__device__ __forceinline__ void kahan_add(V &sum, V &comp, float w, V s) {
+  const V y = vsub(V{w * s.x, w * s.y}, comp);
+  const V t = vadd(sum, y);
+  comp = vsub(vsub(t, sum), y);
   sum = t;
 }
 
 __device__ __forceinline__ void rebase(const ScenarioDev &s, RayLane &L) {
-  L.ox += static_cast<double>(L.px) - static_cast<double>(L.cpx);
-  L.oy += static_cast<double>(L.py) - static_cast<double>(L.cpy);
-  L.px = L.py = L.cpx = L.cpy = 0.0f;
+  L.ox += static_cast<double>(L.p.x) - static_cast<double>(L.cp.x);
+  L.oy += static_cast<double>(L.p.y) - static_cast<double>(L.cp.y);
+  L.p = L.cp = both(0.0f);
   L.pb = grid_pos(s.bathy, L.ox, L.oy);
   L.pc = s.same_grid ? L.pb : grid_pos(s.current, L.ox, L.oy);
 }
@@ -537,19 +572,19 @@ __device__ __forceinline__ void save_row(const BatchArgs &a, const RayLane &L) {
   const int64_t plane = a.save_cap * a.n_stride;
   float *p = a.saved + static_cast<int64_t>(L.saved) * a.n_stride + L.ray;
   p[0] = static_cast<float>(a.t0 + static_cast<double>(L.step) * a.dt);
-  p[plane] = static_cast<float>(L.ox + (static_cast<double>(L.px) - static_cast<double>(L.cpx)));
-  p[2 * plane] = static_cast<float>(L.oy + (static_cast<double>(L.py) - static_cast<double>(L.cpy)));
-  p[3 * plane] = L.kx - L.ckx;
-  p[4 * plane] = L.ky - L.cky;
+  p[plane] = static_cast<float>(L.ox + (static_cast<double>(L.p.x) - static_cast<double>(L.cp.x)));
+  p[2 * plane] = static_cast<float>(L.oy + (static_cast<double>(L.p.y) - static_cast<double>(L.cp.y)));
+  p[3 * plane] = L.k.x - L.ck.x;
+  p[4 * plane] = L.k.y - L.ck.y;
 }
 
 __device__ __forceinline__ void finish(const BatchArgs &a, RayLane &L, int status) {
   const int64_t r = L.ray;
   a.end_state[r] = a.t0 + static_cast<double>(L.step) * a.dt;
-  a.end_state[a.n_stride + r] = L.ox + (static_cast<double>(L.px) - static_cast<double>(L.cpx));
-  a.end_state[2 * a.n_stride + r] = L.oy + (static_cast<double>(L.py) - static_cast<double>(L.cpy));
-  a.end_state[3 * a.n_stride + r] = static_cast<double>(L.kx) - static_cast<double>(L.ckx);
-  a.end_state[4 * a.n_stride + r] = static_cast<double>(L.ky) - static_cast<double>(L.cky);
+  a.end_state[a.n_stride + r] = L.ox + (static_cast<double>(L.p.x) - static_cast<double>(L.cp.x));
+  a.end_state[2 * a.n_stride + r] = L.oy + (static_cast<double>(L.p.y) - static_cast<double>(L.cp.y));
+  a.end_state[3 * a.n_stride + r] = static_cast<double>(L.k.x) - static_cast<double>(L.ck.x);
+  a.end_state[4 * a.n_stride + r] = static_cast<double>(L.k.y) - static_cast<double>(L.ck.y);
   a.n_steps[r] = L.step;
   a.n_saved[r] = L.saved;
   a.status[r] = static_cast<uint8_t>(status);
@@ -565,25 +600,17 @@ __device__ __forceinline__ int32_t save_period(const BatchArgs &a) {
                                                           : static_cast<int32_t>(a.decimation);
 }
 
-// A lane's scenario: from the kernel's parameters in the single-scenario
-// builds (MODE 1, 2), else from the device table (MODE 0, 3).
-template <int MODE>
-__device__ __forceinline__ const ScenarioDev &scenario(const BatchArgs &a, int s) {
-  return (MODE == 1 || MODE == 2) ? a.scen0 : a.scen[s];
-}
-
 template <int MODE>
 __device__ __forceinline__ void start(const BatchArgs &a, RayLane &L, int64_t r) {
   L.ray = r;
-  L.scen = ((MODE == 0 || MODE == 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
+  L.scen = ((MODE == 0 || MODE >= 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
                                                          : 0;
   if (L.scen >= a.n_scenarios) L.scen = 0;
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
   L.ox = a.x0[r];
   L.oy = a.y0[r];
-  L.px = L.py = L.cpx = L.cpy = L.ckx = L.cky = 0.0f;
-  L.kx = static_cast<float>(a.kx0[r]);
-  L.ky = static_cast<float>(a.ky0[r]);
+  L.p = L.cp = L.ck = both(0.0f);
+  L.k = V{static_cast<float>(a.kx0[r]), static_cast<float>(a.ky0[r])};
   L.pb = grid_pos(s.bathy, L.ox, L.oy);
   L.pc = s.same_grid ? L.pb : grid_pos(s.current, L.ox, L.oy);
   L.step = 0;
@@ -608,7 +635,7 @@ __device__ __forceinline__ void start(const BatchArgs &a, RayLane &L, int64_t r)
 template <int MODE>
 __device__ __forceinline__ void resume(const BatchArgs &a, RayLane &L, int64_t r) {
   L.ray = r;
-  L.scen = ((MODE == 0 || MODE == 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
+  L.scen = ((MODE == 0 || MODE >= 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
                                                          : 0;
   if (L.scen >= a.n_scenarios) L.scen = 0;
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
@@ -617,8 +644,8 @@ __device__ __forceinline__ void resume(const BatchArgs &a, RayLane &L, int64_t r
   const float4 q = p[1], c = p[2];
   const int4 k = *reinterpret_cast<const int4 *>(p + 3);
   L.ox = o.x; L.oy = o.y;
-  L.px = q.x; L.py = q.y; L.kx = q.z; L.ky = q.w;
-  L.cpx = c.x; L.cpy = c.y; L.ckx = c.z; L.cky = c.w;
+  L.p = V{q.x, q.y}; L.k = V{q.z, q.w};
+  L.cp = V{c.x, c.y}; L.ck = V{c.z, c.w};
   L.step = k.x; L.saved = k.y; L.to_save = k.z; L.to_rebase = k.w;
   L.pb = grid_pos(s.bathy, L.ox, L.oy);
   L.pc = s.same_grid ? L.pb : grid_pos(s.current, L.ox, L.oy);
@@ -655,9 +682,9 @@ __device__ __forceinline__ uint64_t sweep_key(const BatchArgs &a, const Scenario
                                               const RayLane &L) {
   const PackedGrid &g = s.bathy;
   const uint32_t lim = (1u << a.sweep_cell_bits) - 1u;
-  const uint32_t bx = sweep_block(L.ox + (static_cast<double>(L.px) - static_cast<double>(L.cpx)),
+  const uint32_t bx = sweep_block(L.ox + (static_cast<double>(L.p.x) - static_cast<double>(L.cp.x)),
                                   g.x0, g.inv_sp_xd, lim);
-  const uint32_t by = sweep_block(L.oy + (static_cast<double>(L.py) - static_cast<double>(L.cpy)),
+  const uint32_t by = sweep_block(L.oy + (static_cast<double>(L.p.y) - static_cast<double>(L.cp.y)),
                                   g.y0, g.inv_sp_yd, lim);
   return (static_cast<uint64_t>(L.scen) << a.sweep_key_shift) |
          static_cast<uint64_t>(spread_even16(bx) | (spread_even16(by) << 1));
@@ -666,8 +693,8 @@ __device__ __forceinline__ uint64_t sweep_key(const BatchArgs &a, const Scenario
 __device__ __forceinline__ void store_sweep(const BatchArgs &a, const RayLane &L) {
   float4 *p = reinterpret_cast<float4 *>(a.sweep + L.ray);
   *reinterpret_cast<double2 *>(p) = make_double2(L.ox, L.oy);
-  p[1] = make_float4(L.px, L.py, L.kx, L.ky);
-  p[2] = make_float4(L.cpx, L.cpy, L.ckx, L.cky);
+  p[1] = make_float4(L.p.x, L.p.y, L.k.x, L.k.y);
+  p[2] = make_float4(L.cp.x, L.cp.y, L.ck.x, L.ck.y);
   *reinterpret_cast<int4 *>(p + 3) = make_int4(L.step, L.saved, L.to_save, L.to_rebase);
 }
 
@@ -676,18 +703,16 @@ __device__ __forceinline__ void store_sweep(const BatchArgs &a, const RayLane &L
 // same inputs, so the same values and the same first failure).  Taken once
 // per ray at most: the ray ends there.  One stage in a loop: little code.
 template <int MODE, int STAGE>
-__device__ __forceinline__ int step_status(const ScenarioDev &s, RayLane &L, const WarpTile &W,
-                                           float dt, float half) {
-  float k[4], x[4] = {L.px, L.py, L.kx, L.ky};
+__device__ __forceinline__ int step_status(const ScenarioDev &s, const ScenarioDev &t, RayLane &L,
+                                           const WarpTile &W, float dt, float half) {
+  V p = L.p, k = L.k, dp, dk;
 #pragma unroll 1
   for (int st = 0; st < 4; ++st) {
-    const int r = rhs_f32<MODE, true, STAGE>(s, L, W, x[0], x[1], x[2], x[3], k);
+    const int r = rhs_f32<MODE, true, STAGE>(s, t, L, W, p, k, &dp, &dk);
     if (r != BATCH_COMPLETE) return r;
-    const float w = st == 2 ? dt : half;
-    x[0] = fmaf(w, k[0], L.px);
-    x[1] = fmaf(w, k[1], L.py);
-    x[2] = fmaf(w, k[2], L.kx);
-    x[3] = fmaf(w, k[3], L.ky);
+    const V w = both(st == 2 ? dt : half);
+    p = vfma(w, dp, L.p);
+    k = vfma(w, dk, L.k);
   }
   // not reached: the same four stages failed a moment ago.  Ending the ray
   // all the same keeps every ray's step count bounded.
@@ -705,31 +730,31 @@ __device__ __forceinline__ int step_status(const ScenarioDev &s, RayLane &L, con
 template <int MODE, int STAGE>
 __device__ __forceinline__ int advance(const BatchArgs &a, RayLane &L, const WarpTile &W) {
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
+  const ScenarioDev &t = cells_of<MODE>(a, L.scen);  // the records
   // step constants in FP32 from the host (a conversion here would run on the
   // FP64 pipe, and the compiler re-derives such values under register pressure)
   const float dt = a.dt_f;
   const float half = a.half_f;
-  float k[4], sum[4];
-  int fails = rhs_f32<MODE, false, STAGE>(s, L, W, L.px, L.py, L.kx, L.ky, k);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) sum[q] = k[q];
-  if (STAGE == 2) load_ahead<MODE>(s, L, k[0], k[1]);
-  fails |= rhs_f32<MODE, false, STAGE>(s, L, W, fmaf(half, k[0], L.px), fmaf(half, k[1], L.py),
-                                fmaf(half, k[2], L.kx), fmaf(half, k[3], L.ky), k);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) sum[q] = fmaf(2.0f, k[q], sum[q]);
-  fails |= rhs_f32<MODE, false, STAGE>(s, L, W, fmaf(half, k[0], L.px), fmaf(half, k[1], L.py),
-                                fmaf(half, k[2], L.kx), fmaf(half, k[3], L.ky), k);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) sum[q] = fmaf(2.0f, k[q], sum[q]);
-  fails |= rhs_f32<MODE, false, STAGE>(s, L, W, fmaf(dt, k[0], L.px), fmaf(dt, k[1], L.py),
-                                fmaf(dt, k[2], L.kx), fmaf(dt, k[3], L.ky), k);
-  if (fails != BATCH_COMPLETE) return step_status<MODE, STAGE>(s, L, W, dt, half);
-  const float sixth = a.sixth_f;
-  kahan_add(L.px, L.cpx, sixth * (sum[0] + k[0]));
-  kahan_add(L.py, L.cpy, sixth * (sum[1] + k[1]));
-  kahan_add(L.kx, L.ckx, sixth * (sum[2] + k[2]));
-  kahan_add(L.ky, L.cky, sixth * (sum[3] + k[3]));
+  const V two = both(2.0f);
+  const V hv = both(half), dv = both(dt);
+  V dp, dk, sp, sk;
+  int fails = rhs_f32<MODE, false, STAGE>(s, t, L, W, L.p, L.k, &dp, &dk);
+  sp = dp;
+  sk = dk;
+  if (STAGE == 2) load_ahead<MODE>(s, t, L, dp);
+  fails |= rhs_f32<MODE, false, STAGE>(s, t, L, W, vfma(hv, dp, L.p),
+                                       vfma(hv, dk, L.k), &dp, &dk);
+  sp = vfma(two, dp, sp);
+  sk = vfma(two, dk, sk);
+  fails |= rhs_f32<MODE, false, STAGE>(s, t, L, W, vfma(hv, dp, L.p),
+                                       vfma(hv, dk, L.k), &dp, &dk);
+  sp = vfma(two, dp, sp);
+  sk = vfma(two, dk, sk);
+  fails |= rhs_f32<MODE, false, STAGE>(s, t, L, W, vfma(dv, dp, L.p), vfma(dv, dk, L.k),
+                                       &dp, &dk);
+  if (fails != BATCH_COMPLETE) return step_status<MODE, STAGE>(s, t, L, W, dt, half);
+  kahan_add(L.p, L.cp, a.sixth_f, vadd(sp, dp));
+  kahan_add(L.k, L.ck, a.sixth_f, vadd(sk, dk));
   ++L.step;
   if (--L.to_save == 0) {
     L.to_save = save_period(a);
@@ -750,8 +775,8 @@ template <int MODE>
 __device__ __forceinline__ void tile_refresh(const BatchArgs &a, const RayLane &L, WarpTile &W) {
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
   int cb = 0, ix = 0, iy = 0;
-  float fx, fy;
-  const bool in_grid = L.ray >= 0 && locate(s.bathy, L.pb, L.px, L.py, &cb, &fx, &fy, &ix, &iy);
+  V f;
+  const bool in_grid = L.ray >= 0 && locate<false>(s.bathy, L.pb, L.p, &cb, &f, &ix, &iy);
   const bool in_tile = W.valid && static_cast<unsigned>(ix - W.ti) < kTileCells &&
                        static_cast<unsigned>(iy - W.tj) < kTileCells;
   const unsigned live = __ballot_sync(kFull, in_grid);
@@ -862,25 +887,32 @@ __device__ __forceinline__ void k2_body(const BatchArgs &a) {
 }
 
 // One ray per lane, two builds.  rk4_f32_kernel_1 takes the compiler's
-// register count (~100: 4 blocks of 128 threads, 16 warps, per SM).
-// rk4_f32_kernel_1r is capped at 72 registers (28 warps per SM; 80 B
-// spilled to L1).  The kernel is issue- and latency-bound; when a call has
-// rays for more warps than the first keeps resident, the extra warps hide
-// more of the dependent FP32 chains than the spills cost (4,096^2
-// shelf-slope, 2^20 rays: 30.6 -> 32.7 G ray-steps/s at 128 x 8; caps of
-// 80 / 64 / 56 registers gave 32.0 / 32.7 / 31.5); with fewer rays than
-// lanes the spills only add latency (65,536-ray seamount: 22.2 -> 19.3).
+// register count (80 in mode 2: 6 blocks of 128 threads, 24 warps, per SM).
+// rk4_f32_kernel_1r is capped at 64 registers (32 warps per SM; 100-150 B
+// spilled to L1 in modes 2 and 5).  The kernel is bound by the latency of a
+// step's dependent chain (issue slots 62-65% busy, FP32 and special-function
+// pipes each near half): when a call has rays for more warps than the first
+// keeps resident, the extra warps hide more of it than the spills cost.  Caps
+// of 80 / 72 / 64 / 56, blocks of 128 x 12: 4,096^2 shelf-slope in sweeps,
+// 4.2 M rays x 1,024 steps 44.6 / 43.5 / 43.3 / 53.0 ms; four scenarios, 1 M
+// rays 14.8 / 14.5 / 14.1 / 15.6 ms.  With fewer rays than lanes the spills
+// only add latency.  Moving the origin, compensations and ray index to shared
+// memory instead (no spills at 64) gave 44.2 and 15.5 ms: not kept.
 // The launcher takes the capped build when the launch asks for more blocks
 // per SM than the uncapped one holds.
-// Each comes in four modes: 0 reads the lane's scenario from the device
+// Each comes in modes: 0 reads the lane's scenario from the device
 // table; 1 (one scenario) takes the scenario's fields from the kernel's
 // parameters (operands of the instructions instead of loads at every
 // lookup); 2 is mode 1 and 3 is mode 0 with the current gridded on the
-// bathymetry's grid (every scenario's, for 3).
+// bathymetry's grid (every scenario's, for 3).  Mode 4 is mode 0 for axes of
+// more than 2^22 points (locate, WIDE), in the uncapped builds only.  Mode 5
+// is mode 3 where every scenario has the first one's axes: the geometry is in
+// the kernel's parameters and only a new cell's records go through the table
+// (mode 3 reads ten values of it in each lookup).
 template <int MODE>
 __global__ void __launch_bounds__(256) rk4_f32_kernel_1(BatchArgs a) { k2_body<1, MODE, 0>(a); }
 template <int MODE>
-__global__ void __maxnreg__(72) rk4_f32_kernel_1r(BatchArgs a) { k2_body<1, MODE, 0>(a); }
+__global__ void __maxnreg__(kCappedRegs) rk4_f32_kernel_1r(BatchArgs a) { k2_body<1, MODE, 0>(a); }
 // The sweep form of both: each launch advances its rays by at most
 // sweep_steps steps, the first from their initial states (sweep_first), the
 // later ones from the states the previous launch left.
@@ -889,12 +921,12 @@ __global__ void __launch_bounds__(256) rk4_f32_kernel_1s(BatchArgs a) {
   k2_body<1, MODE, 0, true>(a);
 }
 template <int MODE>
-__global__ void __maxnreg__(72) rk4_f32_kernel_1rs(BatchArgs a) { k2_body<1, MODE, 0, true>(a); }
+__global__ void __maxnreg__(kCappedRegs) rk4_f32_kernel_1rs(BatchArgs a) { k2_body<1, MODE, 0, true>(a); }
 // Two rays per lane hold twice the lane state: no cap.
 template <int MODE>
 __global__ void __launch_bounds__(256) rk4_f32_kernel_2(BatchArgs a) { k2_body<2, MODE, 0>(a); }
 // The tile build (mode 2): one ray per lane (the compiler's register count,
-// 80; capped at 72 it spilled), each warp's tile in dynamic
+// 88), each warp's tile in dynamic
 // shared memory (kTileBytes per warp, then 8 bytes of mbarrier per warp); the
 // arguments stay in the parameter space (__grid_constant__) because the
 // copies read the tensor maps from there.

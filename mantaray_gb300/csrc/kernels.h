@@ -43,16 +43,15 @@ cudaError_t launch_pack_bathy(const BathyDev &b, float4 *cells, cudaStream_t str
 cudaError_t launch_pack_current(const CurrentDev &c, float4 *cells, cudaStream_t stream);
 cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int rays_per_lane,
                            cudaStream_t stream);
-// The integrator build a launch of this shape runs, for n_scenarios
-// scenarios (same_grid: every scenario's current is gridded on its
-// bathymetry's grid; staging: MR_STAGING_*; sweep: the sweep form; null where
-// that build does not exist); a graph's kernel node is found by it.
-const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int n_scenarios,
-                             int same_grid, int staging, int sweep);
+// The integrator build a launch of this shape runs in a mode (batch_mode;
+// staging: MR_STAGING_*; sweep: the sweep form; null where that build does
+// not exist); a graph's kernel node is found by it.
+const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int mode,
+                             int staging, int sweep);
 // Dynamic shared memory of the tile build for blocks of `block` threads.
 size_t rk4_f32_tile_smem(int block);
 // The single-scenario builds (rk4_f32_one.cu): 0 one ray per lane, 1 the same
-// capped at 72 registers, 2 two rays per lane, 3 the tile build, 4 the ahead
+// capped (kCappedRegs), 2 two rays per lane, 3 the tile build, 4 the ahead
 // build (3 and 4: same grid only, else null), 5 and 6 the sweep form of 0
 // and 1.
 const void *rk4_f32_one_function(int build, int same_grid);

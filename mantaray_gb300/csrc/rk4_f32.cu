@@ -5,7 +5,7 @@
 //
 // K2 (rk4_f32_kernel_1 / _1r / _2, device code in k2.cuh): a persistent
 // kernel, grid = SMs x blocks per SM.  Each lane holds 1 or 2 rays (_2); one
-// ray per lane has an uncapped and a 72-register build (_1r), chosen by the
+// ray per lane has an uncapped and a 64-register build (_1r), chosen by the
 // launch shape, and their sweep forms (_1s / _1rs: each launch advances its
 // rays by at most sweep_steps steps, the rays still running re-sorted by
 // position between launches; batch_api.cu queues the sequence).  Each build
@@ -24,6 +24,13 @@
 // `rebase_interval` steps the offset is folded into the FP64 origin, which
 // keeps the offsets (and their rounding) small over tens of thousands of
 // steps.  FP64 is used only for that rebase and for the stored positions.
+//
+// What is the same for x and y, u and v, or kx and ky runs on packed FP32
+// instructions (packed.cuh), and cells are found without conversions (k2.cuh,
+// locate): 319 -> 265 instructions a warp and step on the 65,536-ray seamount.
+// Against the scalar form, bit-identical results: that case, 4,000 steps, 4.90
+// -> 4.45 ms; four scenarios, 1 M rays x 1,000 steps 15.1 -> 13.9 ms; 4,096^2
+// shelf-slope in sweeps, 4.2 M rays x 1,024 steps 45.7 -> 43.3 ms.
 //
 // Memory: each lane keeps the cell records it read last in registers and
 // reuses them while its ray stays in that cell; when the current is gridded
@@ -90,8 +97,10 @@ __global__ void pack_current_cells(CurrentDev cu, float4 *cells) {
   if (ne < cu.u_len && ne < cu.v_len) {
     const double u00 = cu.u[sw], u10 = cu.u[se], u01 = cu.u[nw], u11 = cu.u[ne];
     const double v00 = cu.v[sw], v10 = cu.v[se], v01 = cu.v[nw], v11 = cu.v[ne];
-    r0 = bilinear_coefficients(u00, u10, u01, u11);
-    r1 = bilinear_coefficients(v00, v10, v01, v11);
+    const float4 cu4 = bilinear_coefficients(u00, u10, u01, u11);
+    const float4 cv4 = bilinear_coefficients(v00, v10, v01, v11);
+    r0 = make_float4(cu4.x, cv4.x, cu4.y, cv4.y);
+    r1 = make_float4(cu4.z, cv4.z, cu4.w, cv4.w);
     r2 = make_float4(__double2float_rn((u10 - u00) / cu.xspace),
                      __double2float_rn((u01 - u00) / cu.yspace),
                      __double2float_rn((v10 - v00) / cu.xspace),
@@ -150,40 +159,40 @@ cudaError_t launch_fill_nan(float *p, int64_t count, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// The builds of each table mode: [0] one ray per lane, uncapped; [1] the
-// same capped at 72 registers; [2] two rays per lane; [3] and [4] the sweep
-// form of [0] and [1].  Row 0: mode 0, row 1: mode 3 (every current on its
-// bathymetry's grid).
-static const void *table_builds[2][5] = {
-    {reinterpret_cast<const void *>(&rk4_f32_kernel_1<0>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1r<0>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_2<0>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1s<0>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1rs<0>)},
-    {reinterpret_cast<const void *>(&rk4_f32_kernel_1<3>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1r<3>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_2<3>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1s<3>),
-     reinterpret_cast<const void *>(&rk4_f32_kernel_1rs<3>)}};
+// The builds of a table mode: [0] one ray per lane, uncapped; [1] the same
+// capped at kCappedRegs registers; [2] two rays per lane; [3] and [4] the sweep form of
+// [0] and [1].
+template <int MODE>
+static const void *table_build(int k) {
+  static const void *builds[5] = {reinterpret_cast<const void *>(&rk4_f32_kernel_1<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1r<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_2<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1s<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1rs<MODE>)};
+  return builds[k];
+}
 
 // Resident blocks per SM of each mode's uncapped one-ray build (plain and
 // sweep form) by block size (multiples of 32 up to 256), queried once; 0:
 // not yet known.
-static std::atomic<int> g_resident_1[2][4][9];
+static std::atomic<int> g_resident_1[2][6][9];
 
 size_t rk4_f32_tile_smem(int block) {
   return static_cast<size_t>(block / 32) * (kTileBytes + 8);
 }
 
-const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int n_scenarios,
-                             int same_grid, int staging, int sweep) {
-  const int mode = n_scenarios == 1 ? (same_grid ? 2 : 1) : (same_grid ? 3 : 0);
+const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int mode,
+                             int staging, int sweep) {
+  if (mode == 4)  // results do not depend on the shape or the staging
+    return sweep ? reinterpret_cast<const void *>(&rk4_f32_kernel_1s<4>)
+                 : reinterpret_cast<const void *>(&rk4_f32_kernel_1<4>);
   if (sweep && (staging != 0 || rays_per_lane != 1)) return nullptr;
   if (staging == 1) return (mode == 2 && rays_per_lane == 1) ? rk4_f32_one_function(3, 1) : nullptr;
   if (staging == 2) {
     if (rays_per_lane != 1) return nullptr;
     if (mode == 2) return rk4_f32_one_function(4, 1);
     if (mode == 3) return reinterpret_cast<const void *>(&rk4_f32_kernel_1a<3>);
+    if (mode == 5) return reinterpret_cast<const void *>(&rk4_f32_kernel_1a<5>);
     return nullptr;
   }
   // [0] uncapped, [1] capped, [2] two rays per lane; the sweep form of [0]
@@ -193,8 +202,10 @@ const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, in
   const int sw = sweep ? 1 : 0;
   const void *fn[3];
   for (int k = 0; k < 3; ++k)
-    fn[k] = (mode == 1 || mode == 2) ? rk4_f32_one_function(kOneBuild[sw][k], mode == 2)
-                                     : table_builds[mode == 3][kTableBuild[sw][k]];
+    fn[k] = mode == 1 || mode == 2 ? rk4_f32_one_function(kOneBuild[sw][k], mode == 2)
+             : mode == 5            ? table_build<5>(kTableBuild[sw][k])
+             : mode == 3            ? table_build<3>(kTableBuild[sw][k])
+                                    : table_build<0>(kTableBuild[sw][k]);
   if (rays_per_lane == 2) return fn[2];
   const int slot = (block >= 32 && block <= 256 && block % 32 == 0) ? block / 32 : 0;
   int resident = slot ? g_resident_1[sw][mode][slot].load(std::memory_order_relaxed) : 0;
@@ -220,10 +231,11 @@ cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>(sms * blocks_per_sm);
   void *args[] = {const_cast<BatchArgs *>(&a)};
-  const void *fn = rk4_f32_function(rays_per_lane, block, blocks_per_sm, a.n_scenarios,
-                                    a.all_same_grid, a.staging, a.sweep_steps > 0);
+  const void *fn = rk4_f32_function(rays_per_lane, block, blocks_per_sm, a.mode, a.staging,
+                                    a.sweep_steps > 0);
   if (!fn) return cudaErrorInvalidValue;
-  const size_t smem = a.staging == 1 ? rk4_f32_tile_smem(block)
+  const size_t smem = a.mode == 4 ? 0
+                      : a.staging == 1 ? rk4_f32_tile_smem(block)
                       : a.staging == 2 ? static_cast<size_t>(block) * 80 : 0;
   return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, stream);
 }

@@ -21,12 +21,9 @@
 // gradients below 2^20.  Everything else, NaN and infinities included, is
 // left to the FP64 form (ray_exact.cuh).
 //
-// What is the same for x and y runs on packed instructions (f32x2: two
-// floats in one 64-bit register, the rate of two instructions in the issue
-// slot of one); packed and scalar operations round alike.  ptxas contracts a
-// packed product and a packed sum into one FMA even under -fmad=false: here
-// every product that meets a sum is exact (by a power of two or -1) or is in
-// a written FMA.
+// What is the same for x and y runs on packed instructions (packed.cuh);
+// every product there that meets a sum is exact (by a power of two or -1) or
+// in a written FMA.
 //
 // Host and device code: the host build is what the CPU tests check against
 // 64-bit and wider arithmetic.  -fmad=false / -ffp-contract=off: every fused
@@ -38,6 +35,7 @@
 
 #include "bits.h"
 #include "exp_table.h"
+#include "packed.cuh"
 
 namespace mr {
 
@@ -144,41 +142,8 @@ MR_HD F2 rcp2(F2 x) {
 
 // ---------------------------------------------- two lanes at once (x, y) --
 
-struct V { float x, y; };
 struct V2 { V h, l; };  // a pair (F2) for each of x and y
 
-#if defined(__CUDA_ARCH__)
-#define MR_PACKED(name, op)                                                       \
-  MR_HD V name(V a, V b) {                                                        \
-    unsigned long long p, q, r;                                                   \
-    V o;                                                                          \
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a.x), "f"(a.y));                  \
-    asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(b.x), "f"(b.y));                  \
-    asm(op ".rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(p), "l"(q));                   \
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));                 \
-    return o;                                                                     \
-  }
-MR_PACKED(vadd, "add")
-MR_PACKED(vsub, "sub")
-MR_PACKED(vmul, "mul")
-#undef MR_PACKED
-MR_HD V vfma(V a, V b, V c) {
-  unsigned long long p, q, r, t;
-  V o;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(b.x), "f"(b.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(c.x), "f"(c.y));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(p), "l"(q), "l"(r));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(t));
-  return o;
-}
-#else
-MR_HD V vadd(V a, V b) { return V{a.x + b.x, a.y + b.y}; }
-MR_HD V vsub(V a, V b) { return V{a.x - b.x, a.y - b.y}; }
-MR_HD V vmul(V a, V b) { return V{a.x * b.x, a.y * b.y}; }
-MR_HD V vfma(V a, V b, V c) { return V{fma32(a.x, b.x, c.x), fma32(a.y, b.y, c.y)}; }
-#endif
-MR_HD V both(float a) { return V{a, a}; }
 MR_HD V2 both(F2 a) { return V2{both(a.h), both(a.l)}; }
 MR_HD F2 x_of(V2 a) { return F2{a.h.x, a.l.x}; }
 MR_HD F2 y_of(V2 a) { return F2{a.h.y, a.l.y}; }

@@ -59,7 +59,7 @@ fn build_library(root: &Path, out: &Path) -> PathBuf {
         objects.push(obj);
     }
     for header in ["batch.h", "batch_handle.h", "bits.h", "dispersion.cuh", "exp_table.h", "fields.h", "handles.h",
-                   "k2.cuh", "kernels.h", "lookup.cuh", "netcdf3.h", "ray_exact.cuh", "split.cuh",
+                   "k2.cuh", "kernels.h", "lookup.cuh", "netcdf3.h", "packed.cuh", "ray_exact.cuh", "split.cuh",
                    "split_lookup.cuh", "trig_table.h"] {
         println!("cargo:rerun-if-changed={}", csrc.join(header).display());
     }
