@@ -40,6 +40,7 @@ UNITS = {
     "batch_api.cu": [],
     "batch_static.cu": [],
     "diff.cu": [],
+    "diff_split.cu": ["-fmad=false"],
     "order.cu": [],
     "seed.cu": ["-fmad=false"],
 }

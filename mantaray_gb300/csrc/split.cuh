@@ -94,7 +94,9 @@ MR_HD F2 scale(float p2, F2 a) { return F2{p2 * a.h, p2 * a.l}; }  // p2: a powe
 // Sums and products leave their low half unrounded into the high one (|l| up
 // to a few ulps of h): the operations below lose a.l b.l only, 2^-45 of the
 // product, and the rounding steps saved are a third of the instructions and
-// of the dependent chain.
+// of the dependent chain.  MR_SPLIT_LOW_PRODUCT keeps a.l b.l, for a unit
+// whose results carry products' errors on (diff_split.cu; the trajectories
+// gain nothing from it).
 MR_HD F2 add(F2 a, F2 b) {
   const F2 s = two_sum(a.h, b.h);
   return F2{s.h, s.l + (a.l + b.l)};
@@ -116,7 +118,11 @@ MR_HD F2 add_small(F2 a, F2 b) {
 }
 MR_HD F2 mul(F2 a, F2 b) {
   const float p = a.h * b.h;
+#ifdef MR_SPLIT_LOW_PRODUCT
+  return F2{p, fma32(a.h, b.h, -p) + fma32(a.h, b.l, fma32(a.l, b.l, a.l * b.h))};
+#else
   return F2{p, fma32(a.h, b.h, -p) + fma32(a.h, b.l, a.l * b.h)};
+#endif
 }
 MR_HD F2 mul_f(F2 a, float b) {
   const float p = a.h * b;
@@ -124,7 +130,11 @@ MR_HD F2 mul_f(F2 a, float b) {
 }
 MR_HD F2 sqr(F2 a) {
   const float p = a.h * a.h;
+#ifdef MR_SPLIT_LOW_PRODUCT
+  return F2{p, fma32(a.h + a.h, a.l, fma32(a.l, a.l, fma32(a.h, a.h, -p)))};
+#else
   return F2{p, fma32(a.h + a.h, a.l, fma32(a.h, a.h, -p))};
+#endif
 }
 // 1/sqrt(x), one Newton step of third order on the guess: e = 1 - x r^2.
 MR_HD F2 rsqrt2(F2 x) {
@@ -171,7 +181,11 @@ MR_HD V2 sub(V2 a, V2 b) {
 MR_HD V2 mul(V2 a, V2 b) {
   const V p = vmul(a.h, b.h);
   const V e = vfma(a.h, b.h, vmul(p, both(-1.0f)));
+#ifdef MR_SPLIT_LOW_PRODUCT
+  return V2{p, vfma(a.l, b.h, vfma(a.h, b.l, vfma(a.l, b.l, e)))};
+#else
   return V2{p, vfma(a.l, b.h, vfma(a.h, b.l, e))};
+#endif
 }
 MR_HD V2 mul_f(V2 a, V b) {
   const V p = vmul(a.h, b);
@@ -195,12 +209,8 @@ MR_HD double f2d_normal(float f) {
   return double_of((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u), u << 29);
 }
 MR_HD double f2d_zero(float f) { return f == 0.0f ? 0.0 : f2d_normal(f); }
-// a.h = 0 gives 0 (a.l is 0 there); what f2d_normal makes of a zero a.l the
-// sum rounds away unless a.h is below 2^-74.
-MR_HD double to_double(F2 a) {
-  const double s = f2d_normal(a.h) + f2d_normal(a.l);
-  return a.h == 0.0f ? 0.0 : s;
-}
+// Either half may be 0 (a difference can be all low half).
+MR_HD double to_double(F2 a) { return f2d_zero(a.h) + f2d_zero(a.l); }
 // v = h + m + r exactly: the top 24 bits, the next 23 and the last 6 (for
 // magnitudes outside 2^-73..2^126, zero among them, h = (float)v alone).
 MR_HD void split3(double v, float *h, float *m, float *r) {

@@ -23,6 +23,7 @@ const UNITS: &[(&str, &[&str])] = &[
     ("batch_api.cu", &[]),
     ("batch_static.cu", &[]),
     ("diff.cu", &[]),
+    ("diff_split.cu", &["-fmad=false"]),
     ("order.cu", &[]),
     ("seed.cu", &["-fmad=false"]),
 ];
@@ -58,7 +59,8 @@ fn build_library(root: &Path, out: &Path) -> PathBuf {
             .arg("-o").arg(&obj));
         objects.push(obj);
     }
-    for header in ["batch.h", "batch_handle.h", "bits.h", "dispersion.cuh", "exp_table.h", "fields.h", "handles.h",
+    for header in ["batch.h", "batch_handle.h", "bits.h", "diff.cuh", "diff_split.h",
+                   "dispersion.cuh", "exp_table.h", "fields.h", "handles.h",
                    "k2.cuh", "kernels.h", "lookup.cuh", "netcdf3.h", "packed.cuh", "ray_exact.cuh", "split.cuh",
                    "split_lookup.cuh", "trig_table.h"] {
         println!("cargo:rerun-if-changed={}", csrc.join(header).display());
