@@ -32,9 +32,9 @@
 // flush the same cell.  The per-cell accumulation runs in the working
 // precision; only the accumulation onto the node arrays is FP64.
 //
-// The FP64 forward and adjoint run on float pairs where diff_split.cu covers
-// the call; the kernels here in double serve the rest (few ray-steps for the
-// grid, a stream under capture, grids beyond its limits).
+// In FP64 all three run on float pairs where diff_split.cu covers the call; the
+// kernels here in double serve the rest (few ray-steps for the grid, a stream
+// under capture, grids beyond its limits).
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -261,6 +261,8 @@ DiffCall split_call(const DiffArgs<double> &A) {
   c.ckpt = A.ckpt; c.end_state = A.end_state; c.status = A.status;
   c.grad_end = A.grad_end; c.seg = A.seg; c.grad_state0 = A.grad_state0;
   c.grad_depth = A.grad_depth; c.grad_u = A.grad_u; c.grad_v = A.grad_v;
+  c.dstate0 = A.dstate0; c.d_depth = A.d_depth; c.d_u = A.d_u; c.d_v = A.d_v;
+  c.d_end = A.d_end;
   return c;
 }
 
@@ -387,6 +389,9 @@ int mr_diff_tangent(int precision, const mr_diff_grid *bgrid, const void *depth,
     A.end_state = static_cast<double *>(end_state);
     A.d_end = static_cast<double *>(d_end);
     A.status = status;
+    cudaError_t se = cudaSuccess;
+    if (mr::launch_diff_split(mr::DIFF_TANGENT, mr::split_call(A), s, &se))
+      return se == cudaSuccess ? MR_OK : cuda_fail(se, "diff_tangent launch");
     mr::diff_tangent_kernel<double><<<mr::blocks_for(n), mr::kDiffBlock, 0, s>>>(A);
   } else if (precision == 32) {
     mr::DiffArgs<float> A;

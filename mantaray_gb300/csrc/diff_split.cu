@@ -1,33 +1,38 @@
 // diff_split.cu -- the FP64 differentiation form (forward with checkpoints,
-// adjoint; model and derivations in diff.cu) on float pairs.
+// adjoint, tangent-linear; model and derivations in diff.cu) on float pairs.
 //
 // GB300's FP64 pipe issues 2 lanes per SM and clock and takes 64 cycles an
 // operation, so the FP64 kernels of diff.cu keep it 70% busy with 8% of the
 // issue slots used.  Here the stages run on pairs of floats (split.cuh), with
 // one FP64 anchor a step for each quantity whose error would otherwise add up
 // along the ray:
-//   x, y:          as in split.cuh: the first stage's derivative in FP64, the
-//                  stages' differences from it in pairs;
-//   d(x)/d(k):     M = d(c_g k/|k|)/dk, the term by which the position adjoint
-//                  feeds the wavenumber adjoint at every step, in FP64 at one
-//                  state of the step, the stages' differences from it in pairs;
-//   all the rest   (wavenumber increments, refraction and current terms) is a
-//                  small part per step of what it is added to in FP64, and is
+//   the state:     as x, y in split.cuh: the first stage's derivative in FP64,
+//                  the stages' differences from it in pairs;
+//   d(x)/d(k):     M = d(c_g k/|k|)/dk, the term by which a wavenumber tangent
+//                  (position adjoint) feeds the position tangent (wavenumber
+//                  adjoint) at every step, in FP64 at one state of the step,
+//                  the stages' differences from it in pairs;
+//   all the rest   (refraction and current terms of the tangent and adjoint) is
+//                  a small part per step of what it is added to in FP64, and is
 //                  taken from the pairs, with the product of the low halves
 //                  kept (MR_SPLIT_LOW_PRODUCT: 7% of the time; without it the
 //                  gradients' error after 300 steps is 1.7 times FP64's).
 //
 // 32,768 rays x 300 steps on 512 x 512 nodes, forward and adjoint: 44.0 ms in
-// FP64, 13.6 ms here.  The recomputed forward pass and the adjoint are 2,760
-// and 7,300 instructions a warp-step, two warps a scheduler: what is left is
-// the latency of dependent FP32 operations (2.3 of 4.6 cycles an instruction),
-// and the lanes of a warp in deep and in shallower water (22.5 of 32 active).
-// The variant with FP64 equations in the reverse pass took 17.8 ms.
+// FP64, 14.2 ms here (13.6 with the wavenumbers' derivative in pairs alone,
+// whose error under strong refraction, depths 200 times apart in neighbouring
+// cells, was 6 times FP64's).  The recomputed forward pass and the adjoint are
+// 2,800 and 7,300 instructions a warp-step, two warps a scheduler: what is left
+// is the latency of dependent FP32 operations (2.3 of 4.6 cycles an
+// instruction), and the lanes of a warp in deep and in shallower water (22.5 of
+// 32 active).  The variant with FP64 equations in the reverse pass took 17.8 ms.
+// Tangent-linear, 8,192 rays x 500 steps: 16.2 ms in FP64, 5.3 here, one warp a
+// scheduler.
 // Error against 128-bit arithmetic over 50 to 400 steps of 1 to 4 s on 200 to
 // 600 nodes a side, norm over norm, as a fraction of the FP64 kernels' error
-// (geometric mean of 8 cases): end positions and wavenumbers 0.98, gradients
-// by initial position 0.56, wavenumber 0.74, depth 0.82, u 1.07 (2.4e-15 at
-// 50 steps), v 0.98.
+// (geometric mean of 8 cases): end positions and wavenumbers 0.97, gradients
+// by initial position 0.56, wavenumber 0.74, depth 0.82, u 1.06 (2.4e-15 at
+// 50 steps), v 0.96; tangents of position 0.75, of wavenumber 0.82.
 //
 // With a = kh, N = 2a / sinh 2a, C = 2a coth 2a, I = 1 / sinh 2a and sigma =
 // sqrt(g k tanh a) (identities of the definitions):
@@ -80,42 +85,56 @@ struct SplitArgs {
   F2 dt2, half2, sixth2;
 };
 
-__global__ void build_diff_records(SplitArgs S, float4 *b, double2 *b64, float4 *c, double2 *c64) {
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t bn = static_cast<int64_t>(S.b.nx - 1) * (S.b.ny - 1);
-  const int64_t cn = static_cast<int64_t>(S.c.nx - 1) * (S.c.ny - 1);
-  auto coefficients = [](const double *a, int nx, int64_t cell, double o[4]) {
-    const int64_t base = cell / (nx - 1) * nx + cell % (nx - 1);
-    const double v00 = a[base], v10 = a[base + 1], v01 = a[base + nx], v11 = a[base + nx + 1];
-    o[0] = v00;
-    o[1] = v10 - v00;
-    o[2] = v01 - v00;
-    o[3] = ((v11 - v10) - v01) + v00;
-  };
-  double o[4], p[4];
-  if (k < bn) {
-    coefficients(S.A.bg.a, S.b.nx, k, o);
-    F2 q[4];
-    for (int t = 0; t < 4; ++t) q[t] = to_pair(o[t]);
-    b[2 * k] = make_float4(q[0].h, q[1].h, q[2].h, q[3].h);
-    b[2 * k + 1] = make_float4(q[0].l, q[1].l, q[2].l, q[3].l);
+// Cell `cell`'s bilinear coefficients of nodes a, times u.
+__device__ __forceinline__ void coefficients(const double *a, int nx, int64_t cell, double u,
+                                             double o[4]) {
+  const int64_t base = cell / (nx - 1) * nx + cell % (nx - 1);
+  const double v00 = u * a[base], v10 = u * a[base + 1], v01 = u * a[base + nx],
+               v11 = u * a[base + nx + 1];
+  o[0] = v00;
+  o[1] = v10 - v00;
+  o[2] = v01 - v00;
+  o[3] = ((v11 - v10) - v01) + v00;
+}
+
+// A bathymetry's (current's) cell as pairs, and in FP64 where b64 (c64) is
+// given.  A null u or v counts as zero.
+__device__ __forceinline__ void bathy_record(const double *a, int nx, int64_t k, double unit,
+                                             float4 *b, double2 *b64) {
+  double o[4];
+  coefficients(a, nx, k, unit, o);
+  F2 q[4];
+  for (int t = 0; t < 4; ++t) q[t] = to_pair(o[t]);
+  b[2 * k] = make_float4(q[0].h, q[1].h, q[2].h, q[3].h);
+  b[2 * k + 1] = make_float4(q[0].l, q[1].l, q[2].l, q[3].l);
+  if (b64) {
     b64[2 * k] = make_double2(o[0], o[1]);
     b64[2 * k + 1] = make_double2(o[2], o[3]);
   }
-  if (k < cn) {
-    coefficients(S.A.cg.a, S.c.nx, k, o);
-    coefficients(S.A.cg.b, S.c.nx, k, p);
-    F2 q[4], r[4];
-    for (int t = 0; t < 4; ++t) {
-      q[t] = to_pair(o[t]);
-      r[t] = to_pair(p[t]);
-      c64[4 * k + t] = make_double2(o[t], p[t]);
-    }
-    c[4 * k] = make_float4(q[0].h, r[0].h, q[1].h, r[1].h);
-    c[4 * k + 1] = make_float4(q[2].h, r[2].h, q[3].h, r[3].h);
-    c[4 * k + 2] = make_float4(q[0].l, r[0].l, q[1].l, r[1].l);
-    c[4 * k + 3] = make_float4(q[2].l, r[2].l, q[3].l, r[3].l);
+}
+__device__ __forceinline__ void current_record(const double *u, const double *v, int nx, int64_t k,
+                                               double unit, float4 *c, double2 *c64) {
+  double o[4] = {0.0, 0.0, 0.0, 0.0}, p[4] = {0.0, 0.0, 0.0, 0.0};
+  if (u) coefficients(u, nx, k, unit, o);
+  if (v) coefficients(v, nx, k, unit, p);
+  F2 q[4], r[4];
+  for (int t = 0; t < 4; ++t) {
+    q[t] = to_pair(o[t]);
+    r[t] = to_pair(p[t]);
+    if (c64) c64[4 * k + t] = make_double2(o[t], p[t]);
   }
+  c[4 * k] = make_float4(q[0].h, r[0].h, q[1].h, r[1].h);
+  c[4 * k + 1] = make_float4(q[2].h, r[2].h, q[3].h, r[3].h);
+  c[4 * k + 2] = make_float4(q[0].l, r[0].l, q[1].l, r[1].l);
+  c[4 * k + 3] = make_float4(q[2].l, r[2].l, q[3].l, r[3].l);
+}
+
+__global__ void build_diff_records(SplitArgs S, float4 *b, double2 *b64, float4 *c, double2 *c64) {
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k < static_cast<int64_t>(S.b.nx - 1) * (S.b.ny - 1))
+    bathy_record(S.A.bg.a, S.b.nx, k, 1.0, b, b64);
+  if (k < static_cast<int64_t>(S.c.nx - 1) * (S.c.ny - 1))
+    current_record(S.A.cg.a, S.A.cg.b, S.c.nx, k, 1.0, c, c64);
 }
 
 // The cells a lane holds.
@@ -235,7 +254,8 @@ struct Eqs { F2 w, f, qk, qh, fh; };
 
 template <bool PARTIALS>
 __device__ __forceinline__ void eqs_of(const Wave &wv, F2 h, Eqs *e, bool anchor, double kx,
-                                       double ky, double hd, double *w64, double *beta64) {
+                                       double ky, double hd, double *w64, double *beta64,
+                                       double *f64 = nullptr) {
   const F2 kC2 = F2{0x1.90b41p+1f, 0x1.a0fe04p-24f};  // sqrt(9.8)
   const F2 a = mul(wv.k, h);
   if (a.h > 22.0f) {
@@ -252,6 +272,7 @@ __device__ __forceinline__ void eqs_of(const Wave &wv, F2 h, Eqs *e, bool anchor
       const double w2 = wd * wd;
       const double c = fma(-quarter_of(w2 * w2), k2d * k2d * k2d, 0.25);
       *w64 = kHalfSqrtG * fma(wd, c, wd);
+      if (f64) *f64 = 0.0;
       if (PARTIALS) {
         const double r0 = to_double(wv.rk);
         const double r2 = r0 * r0;  // 1/k^2 to 2^-45: one correction
@@ -303,7 +324,9 @@ __device__ __forceinline__ void eqs_of(const Wave &wv, F2 h, Eqs *e, bool anchor
     const double kRd = kd * (rhod * rhod);
     const double Nd = 4.0 * ad * (Ed * kRd);
     const double rk2d = rkd * rkd;
-    const double s2d = kHalfSqrtG * (km * rhod) * rk2d;
+    const double sgd = kHalfSqrtG * (km * rhod);   // sigma / 2
+    const double s2d = sgd * rk2d;
+    if (f64) *f64 = -4.0 * (kd * sgd) * (Ed * kRd);
     *w64 = fma(s2d, Nd, s2d);
     if (PARTIALS) {
       const double one_cd = fma(-2.0 * ad, fma(Ed, Ed, 1.0) * kRd, 1.0);
@@ -327,21 +350,44 @@ __device__ __forceinline__ void derivative(const SplitArgs &S, const DiffCell &C
 
 __device__ __forceinline__ V2 lanes(F2 a, F2 b) { return V2{V{a.h, b.h}, V{a.l, b.l}}; }
 
-// FP64 fields at the base point: depth, and depth, u, v.
+// FP64 fields at the base point: depth, and all of them.
 __device__ __forceinline__ double depth64(const SplitArgs &S, const Base &b) {
   const double2 *p = S.b.rec64 + static_cast<int64_t>(b.j * (S.b.nx - 1) + b.i) * 2;
   const double2 p0 = __ldg(p), p1 = __ldg(p + 1);
   return fma(b.fy, fma(b.fx, p1.y, p1.x), fma(b.fx, p0.y, p0.x));
 }
+struct Fields64 {
+  double h, u, v;            // at the point
+  double gx, gy;             // depth's cell gradient
+  double ux, uy, vx, vy;     // (u, v)'s
+};
 template <bool SAME>
-__device__ __forceinline__ void fields64(const SplitArgs &S, const Base &b, const Base &c,
-                                         double *h, double *u, double *v) {
-  *h = depth64(S, b);
+__device__ __forceinline__ Fields64 fields64(const SplitArgs &S, const Base &b, const Base &c) {
+  const double2 *p = S.b.rec64 + static_cast<int64_t>(b.j * (S.b.nx - 1) + b.i) * 2;
+  const double2 p0 = __ldg(p), p1 = __ldg(p + 1);
   const Base &g = SAME ? b : c;
   const double2 *q = S.c.rec64 + static_cast<int64_t>(g.j * (S.c.nx - 1) + g.i) * 4;
   const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
-  *u = fma(g.fy, fma(g.fx, q3.x, q2.x), fma(g.fx, q1.x, q0.x));
-  *v = fma(g.fy, fma(g.fx, q3.y, q2.y), fma(g.fx, q1.y, q0.y));
+  Fields64 f;
+  f.h = fma(b.fy, fma(b.fx, p1.y, p1.x), fma(b.fx, p0.y, p0.x));
+  f.u = fma(g.fy, fma(g.fx, q3.x, q2.x), fma(g.fx, q1.x, q0.x));
+  f.v = fma(g.fy, fma(g.fx, q3.y, q2.y), fma(g.fx, q1.y, q0.y));
+  f.gx = p0.y * S.b.inv_dx;
+  f.gy = p1.x * S.b.inv_dy;
+  f.ux = q1.x * S.c.inv_dx;
+  f.vx = q1.y * S.c.inv_dx;
+  f.uy = q2.x * S.c.inv_dy;
+  f.vy = q2.y * S.c.inv_dy;
+  return f;
+}
+
+// The right-hand side at the base point in FP64.
+__device__ __forceinline__ void anchors(const Fields64 &F, const double y[4], double w, double f,
+                                        double a[4]) {
+  a[0] = fma(w, y[2], F.u);
+  a[1] = fma(w, y[3], F.v);
+  a[2] = fma(f, F.gx, -fma(y[2], F.ux, y[3] * F.vx));
+  a[3] = fma(f, F.gy, -fma(y[2], F.uy, y[3] * F.vy));
 }
 
 // The stage point at displacement disp and wavenumber kv; false outside.
@@ -373,14 +419,18 @@ __device__ __forceinline__ bool forward_step(const SplitArgs &S, DiffCell &C, co
   const V2 k = lanes(to_pair(y[2]), to_pair(y[3]));
   Wave wv = wave_of(k);
   bool ok = diff_ok(p, wv.k2.h);
-  double h64, u64, v64, w64;
-  fields64<SAME>(S, b, c, &h64, &u64, &v64);
+  double w64, f64;
   Eqs e;
-  eqs_of<false>(wv, p.h, &e, true, y[2], y[3], h64, &w64, nullptr);
   V2 d1, d, dk;
+  double a[4];
+  {
+    const Fields64 F = fields64<SAME>(S, b, c);
+    eqs_of<false>(wv, p.h, &e, true, y[2], y[3], F.h, &w64, nullptr, &f64);
+    anchors(F, y, w64, f64, a);
+  }
   derivative(S, C, wv, p, e, &d1, &dk);
-  const double ax = fma(w64, y[2], u64), ay = fma(w64, y[3], v64);
-  V2 sd = zero2(), sk = dk;
+  const V2 k1 = dk;
+  V2 sd = zero2(), sk = sd;
   d = d1;
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {
@@ -395,14 +445,14 @@ __device__ __forceinline__ bool forward_step(const SplitArgs &S, DiffCell &C, co
     derivative(S, C, wv, p, e, &d, &dk);
     const float wt = st == 2 ? 1.0f : 2.0f;
     sd = add(sd, scale(wt, sub(d, d1)));
-    sk = add(sk, scale(wt, dk));
+    sk = add(sk, scale(wt, sub(dk, k1)));
   }
   if (!ok) return false;
-  const V2 s6 = mul(sd, both(S.sixth2));
-  yn[0] = y[0] + (fma(S.A.dt, ax, f2d_zero(s6.h.x)) + f2d_zero(s6.l.x));
-  yn[1] = y[1] + (fma(S.A.dt, ay, f2d_zero(s6.h.y)) + f2d_zero(s6.l.y));
-  yn[2] = fma(S.sixth, to_double(x_of(sk)), y[2]);
-  yn[3] = fma(S.sixth, to_double(y_of(sk)), y[3]);
+  const V2 s6 = mul(sd, both(S.sixth2)), k6 = mul(sk, both(S.sixth2));
+  yn[0] = y[0] + (fma(S.A.dt, a[0], f2d_zero(s6.h.x)) + f2d_zero(s6.l.x));
+  yn[1] = y[1] + (fma(S.A.dt, a[1], f2d_zero(s6.h.y)) + f2d_zero(s6.l.y));
+  yn[2] = y[2] + (fma(S.A.dt, a[2], f2d_zero(k6.h.x)) + f2d_zero(k6.l.x));
+  yn[3] = y[3] + (fma(S.A.dt, a[3], f2d_zero(k6.h.y)) + f2d_zero(k6.l.y));
   return true;
 }
 
@@ -451,10 +501,31 @@ __global__ void __launch_bounds__(kSplitBlock, 6)
 
 // ---------------------------------------------------------------- adjoint --
 
+// The adjoint (tangent) state is held in units of 2^e, e the exponent of its
+// largest component at the start (floats reach from 2^-126 to 2^128, gradients
+// can be anything); e = 0 when that is beyond 2^+-900.
+__device__ __forceinline__ uint32_t high_word(double v) {
+  return static_cast<uint32_t>(bits_of(v) >> 32) & 0x7fffffffu;
+}
+__device__ __forceinline__ uint32_t largest_word(const double l[4]) {
+  return max(max(high_word(l[0]), high_word(l[1])), max(high_word(l[2]), high_word(l[3])));
+}
+__device__ __forceinline__ uint32_t unit_of(const double l[4]) {
+  const uint32_t e = largest_word(l) >> 20;
+  return (e > 123 && e < 1923 ? e : 1023u) << 20;
+}
+// Whether a step may use the pairs: the largest between 2^-60 and 2^60 units,
+// or all of them zero.
+__device__ __forceinline__ bool in_units(const double l[4]) {
+  const uint32_t w = largest_word(l);
+  const uint64_t any = bits_of(l[0]) | bits_of(l[1]) | bits_of(l[2]) | bits_of(l[3]);
+  return (w > (963u << 20) && w < (1083u << 20)) || (any << 1) == 0;
+}
+
 // Sums of pairs over the stages a ray spends in a cell, exact but for the
 // third words' rounding (as pairs they lost 2^-48 of the sum at every addition:
-// 4.6 times the FP64 kernels' error in the node gradients of u, for 12.6 in
-// place of 13.6 ms).
+// 4.6 times the FP64 kernels' error in the node gradients of u, for 7% less
+// time).
 struct Sum2 {
   V h, l, m;
 };
@@ -619,27 +690,6 @@ __device__ __noinline__ bool anchor_at(const SplitArgs &S, const double *yin, MA
   eqs_of<true>(wv, p.h, &e, true, y[2], y[3], depth64(S, b), &w64, &beta64);
   *M = MAnchor{w64, beta64, y[2], y[3], e.w, beta_of(wv, e), wv.kv};
   return true;
-}
-
-// The adjoint state is held in units of 2^e, e the exponent of its largest
-// component at the start (floats reach from 2^-126 to 2^128, gradients can be
-// anything); e = 0 when that is beyond 2^+-900.
-__device__ __forceinline__ uint32_t high_word(double v) {
-  return static_cast<uint32_t>(bits_of(v) >> 32) & 0x7fffffffu;
-}
-__device__ __forceinline__ uint32_t largest_word(const double l[4]) {
-  return max(max(high_word(l[0]), high_word(l[1])), max(high_word(l[2]), high_word(l[3])));
-}
-__device__ __forceinline__ uint32_t unit_of(const double l[4]) {
-  const uint32_t e = largest_word(l) >> 20;
-  return (e > 123 && e < 1923 ? e : 1023u) << 20;
-}
-// Whether a step may use the pairs: the largest between 2^-60 and 2^60 units,
-// or all of them zero.
-__device__ __forceinline__ bool in_units(const double l[4]) {
-  const uint32_t w = largest_word(l);
-  const uint64_t any = bits_of(l[0]) | bits_of(l[1]) | bits_of(l[2]) | bits_of(l[3]);
-  return (w > (963u << 20) && w < (1083u << 20)) || (any << 1) == 0;
 }
 
 // A step backward in FP64 (diff.cu), its stage states recomputed from y; the
@@ -827,6 +877,228 @@ __global__ void __launch_bounds__(kSplitBlock, 4)
   for (int q = 0; q < 4; ++q) A.grad_state0[q * A.n + i] = lam[q] * acc.unit();
 }
 
+// ---------------------------------------------------------------- tangent --
+
+// The tangent form's own arguments: the tangent fields' records, in the call's
+// unit (null: none), and the high word of that unit, 0 where floats do not
+// hold the tangents (every step then runs in FP64).
+struct TangentArgs {
+  SplitArgs S;
+  const float4 *db, *dc;
+  const uint32_t *unit;
+};
+
+// The largest high word of the tangents given.
+__global__ void largest_tangent(DiffArgs<double> A, uint32_t *word) {
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t bn = static_cast<int64_t>(A.bg.nx) * A.bg.ny;
+  const int64_t cn = static_cast<int64_t>(A.cg.nx) * A.cg.ny;
+  uint32_t w = 0;
+  for (int64_t k = t0; k < 4 * A.n; k += stride) w = max(w, high_word(A.dstate0[k]));
+  if (A.d_depth)
+    for (int64_t k = t0; k < bn; k += stride) w = max(w, high_word(A.d_depth[k]));
+  for (int64_t k = t0; k < cn; k += stride) {
+    if (A.d_u) w = max(w, high_word(A.d_u[k]));
+    if (A.d_v) w = max(w, high_word(A.d_v[k]));
+  }
+  w = __reduce_max_sync(0xffffffffu, w);
+  if ((threadIdx.x & 31) == 0 && w) atomicMax(word, w);
+}
+
+// The unit's high word from the largest one.
+__device__ __forceinline__ uint32_t tangent_unit(uint32_t word) {
+  const uint32_t e = word >> 20;
+  return word == 0 ? 1023u << 20 : e > 123 && e < 1923 ? e << 20 : 0u;
+}
+
+__global__ void build_tangent_records(TangentArgs T, float4 *db, float4 *dc) {
+  const DiffArgs<double> &A = T.S.A;
+  const uint32_t unit = tangent_unit(*T.unit);
+  if (!unit) return;
+  const double per = double_of(0x7fe00000u - unit, 0u);
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (db && k < static_cast<int64_t>(A.bg.nx - 1) * (A.bg.ny - 1))
+    bathy_record(A.d_depth, A.bg.nx, k, per, db, nullptr);
+  if (dc && k < static_cast<int64_t>(A.cg.nx - 1) * (A.cg.ny - 1))
+    current_record(A.d_u, A.d_v, A.cg.nx, k, per, dc, nullptr);
+}
+
+// One stage's tangent of (dx, dk): m = M dk, t = m + the rest, and tk.
+template <bool SAME>
+__device__ __forceinline__ void stage_jvp(const SplitArgs &S, const DiffCell &C, const DiffCell &D,
+                                          bool depth, bool current, const Wave &wv, const At &p,
+                                          const Eqs &e, V2 dx, V2 dk, V2 *m, V2 *t, V2 *tk) {
+  F2 dh = sum_lanes(mul(mul(lanes(p.hx, p.hy), S.b.inv), dx));
+  const V2 dc = mul(dx, S.c.inv);
+  V2 duv = add(mul(p.wx, both(x_of(dc))), mul(p.wy, both(y_of(dc))));
+  At q;
+  if (depth || current) fields_at<SAME>(D, p.fb, p.fc, &q);
+  if (depth) dh = add(dh, q.h);
+  if (current) duv = add(duv, q.uv);
+  const F2 alpha = sum_lanes(mul(wv.kv, dk));
+  const F2 qhr = mul(e.qh, wv.rk);
+  *m = add(mul(both(e.w), dk), mul(both(mul(beta_of(wv, e), alpha)), wv.kv));
+  *t = add(*m, add(mul(both(mul(qhr, dh)), wv.kv), duv));
+  const F2 df = add(mul(e.fh, dh), neg(mul(qhr, alpha)));
+  V2 g = mul(both(df), V2{V{C.b[0].y, C.b[0].z}, V{C.b[1].y, C.b[1].z}});
+  if (depth) g = add(g, mul(both(e.f), V2{V{D.b[0].y, D.b[0].z}, V{D.b[1].y, D.b[1].z}}));
+  F2 tx = sum_lanes(mul(dk, C.wx())), ty = sum_lanes(mul(dk, C.wy()));
+  if (current) {
+    tx = add(tx, sum_lanes(mul(wv.kv, D.wx())));
+    ty = add(ty, sum_lanes(mul(wv.kv, D.wy())));
+  }
+  *tk = sub(mul(g, S.b.inv), mul(lanes(tx, ty), S.c.inv));
+}
+
+// The tangent fields' cells of a stage, those the lane holds in C.
+__device__ __forceinline__ void take_tangent_cells(const TangentArgs &T, const DiffCell &C,
+                                                   DiffCell &D) {
+  if (T.db && D.bkey != C.bkey) {
+    const float4 *p = T.db + static_cast<int64_t>(C.bkey) * 2;
+    D.b[0] = ld4(p);
+    D.b[1] = ld4(p + 1);
+    D.bkey = C.bkey;
+  }
+  if (T.dc && D.ckey != C.ckey) {
+    const float4 *p = T.dc + static_cast<int64_t>(C.ckey) * 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) D.c[q] = ld4(p + q);
+    D.ckey = C.ckey;
+  }
+}
+
+// A step of the state and its tangent; false (y and dy as they were) when a
+// stage is outside the pairs' domain.
+template <bool SAME>
+__device__ __forceinline__ bool tangent_step(const TangentArgs &T, DiffCell &C, DiffCell &D,
+                                             double y[4], double dy[4]) {
+  const SplitArgs &S = T.S;
+  Base b, c;
+  if (!base_of(S.b, y[0], y[1], &b)) return false;
+  if (!SAME && !base_of(S.c, y[0], y[1], &c)) return false;
+  const V2 k = lanes(to_pair(y[2]), to_pair(y[3]));
+  const V2 dx0 = lanes(to_pair(dy[0]), to_pair(dy[1]));
+  const V2 dk0 = lanes(to_pair(dy[2]), to_pair(dy[3]));
+  const bool depth = T.db != nullptr, current = T.dc != nullptr;
+  V2 disp = zero2(), q = k, dx = dx0, dq = dk0;       // the stage's state
+  V2 d1 = disp, k1 = disp, m1 = disp, sd = disp, sk = disp, sdx = disp, sdk = disp;
+  double a[4] = {0.0, 0.0, 0.0, 0.0}, mx = 0.0, my = 0.0;  // anchors
+#pragma unroll 1
+  for (int st = 0; st < 4; ++st) {
+    At p;
+    if (!stage_at<SAME>(S, b, c, disp, C, &p)) return false;
+    take_tangent_cells(T, C, D);
+    const Wave wv = wave_of(q);
+    if (!diff_ok(p, wv.k2.h)) return false;
+    Eqs e;
+    Fields64 F{};
+    double w64 = 0.0, beta64 = 0.0, f64 = 0.0;
+    if (st == 0) F = fields64<SAME>(S, b, c);
+    eqs_of<true>(wv, p.h, &e, st == 0, y[2], y[3], F.h, &w64, &beta64, &f64);
+    V2 d, dk, m, t, tk;
+    derivative(S, C, wv, p, e, &d, &dk);
+    stage_jvp<SAME>(S, C, D, depth, current, wv, p, e, dx, dq, &m, &t, &tk);
+    if (st == 0) {
+      anchors(F, y, w64, f64, a);
+      const double kg = beta64 * fma(y[2], dy[2], y[3] * dy[3]);
+      mx = fma(w64, dy[2], kg * y[2]);
+      my = fma(w64, dy[3], kg * y[3]);
+      d1 = d;
+      m1 = m;
+      k1 = dk;
+      sdx = sub(t, m);
+      sdk = tk;
+    } else {
+      const float wt = st == 3 ? 1.0f : 2.0f;
+      sd = add(sd, scale(wt, sub(d, d1)));
+      sk = add(sk, scale(wt, sub(dk, k1)));
+      sdx = add(sdx, scale(wt, sub(t, m1)));
+      sdk = add(sdk, scale(wt, tk));
+    }
+    const V2 hs = both(st == 2 ? S.dt2 : S.half2);
+    disp = mul(d, hs);
+    q = add(k, mul(dk, hs));
+    dx = add(dx0, mul(t, hs));
+    dq = add(dk0, mul(tk, hs));
+  }
+  const V2 s6 = mul(sd, both(S.sixth2)), k6 = mul(sk, both(S.sixth2));
+  const V2 t6 = mul(sdx, both(S.sixth2));
+  y[0] += fma(S.A.dt, a[0], f2d_zero(s6.h.x)) + f2d_zero(s6.l.x);
+  y[1] += fma(S.A.dt, a[1], f2d_zero(s6.h.y)) + f2d_zero(s6.l.y);
+  y[2] += fma(S.A.dt, a[2], f2d_zero(k6.h.x)) + f2d_zero(k6.l.x);
+  y[3] += fma(S.A.dt, a[3], f2d_zero(k6.h.y)) + f2d_zero(k6.l.y);
+  dy[0] += fma(S.A.dt, mx, f2d_zero(t6.h.x)) + f2d_zero(t6.l.x);
+  dy[1] += fma(S.A.dt, my, f2d_zero(t6.h.y)) + f2d_zero(t6.l.y);
+  dy[2] = fma(S.sixth, to_double(x_of(sdk)), dy[2]);
+  dy[3] = fma(S.sixth, to_double(y_of(sdk)), dy[3]);
+  return true;
+}
+
+// A step in FP64 (diff.cu), state and tangent; false when the ray stops.
+__device__ __noinline__ bool fp64_tangent(const DiffArgs<double> &A, double *y, double *dy) {
+  double t[4], dt[4], sum[4] = {0.0, 0.0, 0.0, 0.0}, dsum[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { t[q] = y[q]; dt[q] = dy[q]; }
+#pragma unroll 1
+  for (int st = 0; st < 4; ++st) {
+    Point<double> P;
+    double k[4], d[4];
+    if (!eval(A, t, P, k)) return false;
+    jvp(A, t, P, dt, d);
+    const double wt = st == 0 || st == 3 ? 1.0 : 2.0, h = st == 2 ? A.dt : A.dt * 0.5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sum[q] = sum[q] + k[q] * wt;
+      dsum[q] = dsum[q] + d[q] * wt;
+      t[q] = y[q] + k[q] * h;
+      dt[q] = dy[q] + d[q] * h;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    y[q] += sum[q] * (A.dt / 6.0);
+    dy[q] += dsum[q] * (A.dt / 6.0);
+  }
+  return true;
+}
+
+template <bool SAME>
+__global__ void __launch_bounds__(kSplitBlock)
+    diff_split_tangent(const __grid_constant__ TangentArgs T) {
+  const DiffArgs<double> &A = T.S.A;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= A.n) return;
+  double y[4] = {A.x0[i], A.y0[i], A.kx0[i], A.ky0[i]};
+  const uint32_t word = tangent_unit(*T.unit);
+  const bool pairs = word != 0;
+  const double unit = pairs ? double_of(word, 0u) : 1.0;
+  const double per = pairs ? double_of(0x7fe00000u - word, 0u) : 1.0;
+  double dy[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) dy[q] = A.dstate0[q * A.n + i] * per;
+  bool ok = true;
+  DiffCell C, D;
+  for (int64_t s = 0; s < A.steps; ++s) {
+    if (!(pairs && in_units(dy) && tangent_step<SAME>(T, C, D, y, dy))) {
+      double yv[4], dv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { yv[q] = y[q]; dv[q] = dy[q] * unit; }
+      ok = fp64_tangent(A, yv, dv);
+      if (!ok) break;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { y[q] = yv[q]; dy[q] = dv[q] * per; }
+    }
+  }
+  const double nan = NAN;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    A.end_state[q * A.n + i] = ok ? y[q] : nan;
+    A.d_end[q * A.n + i] = ok ? dy[q] * unit : nan;
+  }
+  A.status[i] = ok ? 0 : 1;
+}
+
 F2 host_pair(double v) {
   const float h = static_cast<float>(v);
   return F2{h, static_cast<float>(v - static_cast<double>(h))};
@@ -874,6 +1146,8 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   A.ckpt = k.ckpt; A.end_state = k.end_state; A.status = k.status;
   A.grad_end = k.grad_end; A.seg = k.seg; A.grad_state0 = k.grad_state0;
   A.grad_depth = k.grad_depth; A.grad_u = k.grad_u; A.grad_v = k.grad_v;
+  A.dstate0 = k.dstate0; A.d_depth = k.d_depth; A.d_u = k.d_u; A.d_v = k.d_v;
+  A.d_end = k.d_end;
   S.b = field_of(k.bnx, k.bny, k.bx0, k.by0, k.b_inv_dx, k.b_inv_dy);
   S.c = field_of(k.cnx, k.cny, k.cx0, k.cy0, k.c_inv_dx, k.c_inv_dy);
   S.sixth = k.dt / 6.0;
@@ -884,10 +1158,15 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   // while the stream is being captured (the allocation would become a node of
   // the caller's graph).  From the device's own pool, which gives it back at
   // the next synchronisation: 0.2 ms a call for the 50 MB of 512 x 512 cells,
-  // where the kernels are 44 -> 13.6 ms.
+  // where the kernels are 44 -> 14.2 ms.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   char *mem = nullptr;
-  const size_t bytes = static_cast<size_t>(bn) * 64 + static_cast<size_t>(cn) * 128;
+  const bool db = form == DIFF_TANGENT && k.d_depth;
+  const bool dc = form == DIFF_TANGENT && (k.d_u || k.d_v);
+  const size_t records = static_cast<size_t>(bn) * 64 + static_cast<size_t>(cn) * 128;
+  const size_t db_bytes = db ? static_cast<size_t>(bn) * 32 : 0;
+  const size_t dc_bytes = dc ? static_cast<size_t>(cn) * 64 : 0;
+  const size_t bytes = records + db_bytes + dc_bytes + 16;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
       cudaMallocAsync(reinterpret_cast<void **>(&mem), bytes, stream) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -907,11 +1186,25 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
       diff_split_forward<true><<<grid, kSplitBlock, 0, stream>>>(S);
     else
       diff_split_forward<false><<<grid, kSplitBlock, 0, stream>>>(S);
-  } else {
+  } else if (form == DIFF_ADJOINT) {
     if (k.same_grid)
       diff_split_adjoint<true><<<grid, kSplitBlock, 0, stream>>>(S);
     else
       diff_split_adjoint<false><<<grid, kSplitBlock, 0, stream>>>(S);
+  } else {
+    uint32_t *unit = reinterpret_cast<uint32_t *>(mem + records + db_bytes + dc_bytes);
+    float4 *dbr = db ? reinterpret_cast<float4 *>(mem + records) : nullptr;
+    float4 *dcr = dc ? reinterpret_cast<float4 *>(mem + records + db_bytes) : nullptr;
+    const TangentArgs T{S, dbr, dcr, unit};
+    (void)cudaMemsetAsync(unit, 0, sizeof(uint32_t), stream);
+    largest_tangent<<<304, 256, 0, stream>>>(A, unit);
+    if (db || dc)
+      build_tangent_records<<<static_cast<unsigned>((cells + 255) / 256), 256, 0, stream>>>(T, dbr,
+                                                                                            dcr);
+    if (k.same_grid)
+      diff_split_tangent<true><<<grid, kSplitBlock, 0, stream>>>(T);
+    else
+      diff_split_tangent<false><<<grid, kSplitBlock, 0, stream>>>(T);
   }
   *err = cudaGetLastError();
   const cudaError_t f = cudaFreeAsync(mem, stream);

@@ -22,9 +22,11 @@ struct DiffCall {
   uint8_t *status;
   const double *grad_end;
   double *seg, *grad_state0, *grad_depth, *grad_u, *grad_v;
+  const double *dstate0, *d_depth, *d_u, *d_v;
+  double *d_end;
 };
 
-enum DiffForm : int { DIFF_FORWARD = 0, DIFF_ADJOINT = 1 };
+enum DiffForm : int { DIFF_FORWARD = 0, DIFF_ADJOINT = 1, DIFF_TANGENT = 2 };
 
 // Runs the call on pairs; false (nothing queued) when they do not cover it or
 // there is no memory for the records.  *err: the outcome of what was queued.

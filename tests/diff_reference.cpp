@@ -157,3 +157,61 @@ extern "C" void adjoint(const int64_t *nodes, const double *geom, const double *
     gv[i] = (double)V[i];
   }
 }
+
+static void jvp(const Case &C, const Q *s, const Point &p, const Q *ds, const double *dd,
+                const double *du, const double *dv, Q *dF) {
+  Field d{}, u{}, v{};
+  if (dd) d = take(dd, C.g, p.b, p.bx, p.by);
+  if (du) u = take(du, C.c, p.c, p.cx, p.cy);
+  if (dv) v = take(dv, C.c, p.c, p.cx, p.cy);
+  const Q dh = p.h.dx * ds[0] + p.h.dy * ds[1] + d.v, dk = p.c0 * ds[2] + p.s0 * ds[3];
+  const Q k = p.c0 * s[2] + p.s0 * s[3], dw = (p.qk - p.w) / k * dk + p.qh / k * dh;
+  const Q df = p.fk * dk + p.fh * dh;
+  dF[0] = p.w * ds[2] + s[2] * dw + p.u.dx * ds[0] + p.u.dy * ds[1] + u.v;
+  dF[1] = p.w * ds[3] + s[3] * dw + p.v.dx * ds[0] + p.v.dy * ds[1] + v.v;
+  dF[2] = df * p.h.gx + p.f * d.gx - ds[2] * p.u.gx - s[2] * u.gx - ds[3] * p.v.gx - s[3] * v.gx;
+  dF[3] = df * p.h.gy + p.f * d.gy - ds[2] * p.u.gy - s[2] * u.gy - ds[3] * p.v.gy - s[3] * v.gy;
+}
+
+// dd, du, dv: tangent fields or null; dstate, d_end: [4][n].
+extern "C" void tangent(const int64_t *nodes, const double *geom, const double *depth,
+                        const double *u, const double *v, double dt, int64_t steps, int64_t n,
+                        int64_t first, int64_t last, const double *rays, const double *dstate,
+                        const double *dd, const double *du, const double *dv, double *end,
+                        uint8_t *status, double *d_end) {
+  const Case C = make(nodes, geom, depth, u, v, dt, steps, n);
+  for (int64_t r = first; r < last; ++r) {
+    Q y[4], dy[4], F[4], dF[4], t[4], d[4], sum[4], dsum[4];
+    Point p;
+    bool ok = true;
+    for (int q = 0; q < 4; ++q) {
+      y[q] = rays[q * n + r];
+      dy[q] = dstate[q * n + r];
+    }
+    for (int64_t s = 0; s < steps && ok; ++s) {
+      for (int st = 0; st < 4 && ok; ++st) {
+        for (int q = 0; q < 4; ++q) {
+          const Q h = st == 3 ? C.dt : C.dt / 2;
+          t[q] = st == 0 ? y[q] : y[q] + F[q] * h;
+          d[q] = st == 0 ? dy[q] : dy[q] + dF[q] * h;
+        }
+        ok = eval(C, t, &p, F);
+        if (ok) jvp(C, t, p, d, dd, du, dv, dF);
+        for (int q = 0; q < 4; ++q) {
+          const Q wt = st == 0 || st == 3 ? 1 : 2;
+          sum[q] = (st == 0 ? 0 : sum[q]) + wt * F[q];
+          dsum[q] = (st == 0 ? 0 : dsum[q]) + wt * dF[q];
+        }
+      }
+      for (int q = 0; q < 4; ++q) {
+        y[q] += sum[q] * C.dt / 6;
+        dy[q] += dsum[q] * C.dt / 6;
+      }
+    }
+    status[r] = !ok;
+    for (int q = 0; q < 4; ++q) {
+      end[q * n + r] = ok ? (double)y[q] : NAN;
+      d_end[q * n + r] = ok ? (double)dy[q] : NAN;
+    }
+  }
+}
