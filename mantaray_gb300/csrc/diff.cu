@@ -56,12 +56,13 @@ __global__ void __launch_bounds__(64) diff_forward_kernel(DiffArgs<T> A) {
   if (i >= A.n) return;
   T y[4] = {A.x0[i], A.y0[i], A.kx0[i], A.ky0[i]};
   bool ok = true;
+  Held<T> N;
   for (int64_t s = 0; s < A.steps; ++s) {
     if (s % A.ck_every == 0) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) A.ckpt[((s / A.ck_every) * 4 + q) * A.n + i] = y[q];
     }
-    if (!rk4(A, y)) {
+    if (!rk4(A, y, N)) {
       ok = false;
       break;
     }
@@ -79,23 +80,24 @@ __global__ void __launch_bounds__(64) diff_tangent_kernel(DiffArgs<T> A) {
   T y[4] = {A.x0[i], A.y0[i], A.kx0[i], A.ky0[i]};
   T dy[4] = {A.dstate0[i], A.dstate0[A.n + i], A.dstate0[2 * A.n + i], A.dstate0[3 * A.n + i]};
   bool ok = true;
+  Held<T> N;
   const T half = A.dt * T(0.5), sixth = A.dt / T(6);
   for (int64_t s = 0; s < A.steps && ok; ++s) {
     Point<T> P;
     T k1[4], k2[4], k3[4], k4[4], d1[4], d2[4], d3[4], d4[4], t[4], dt_[4];
-    ok = eval(A, y, P, k1);
+    ok = eval(A, y, P, k1, N);
     if (ok) jvp(A, y, P, dy, d1);
 #pragma unroll
     for (int q = 0; q < 4; ++q) { t[q] = y[q] + k1[q] * half; dt_[q] = dy[q] + d1[q] * half; }
-    ok = ok && eval(A, t, P, k2);
+    ok = ok && eval(A, t, P, k2, N);
     if (ok) jvp(A, t, P, dt_, d2);
 #pragma unroll
     for (int q = 0; q < 4; ++q) { t[q] = y[q] + k2[q] * half; dt_[q] = dy[q] + d2[q] * half; }
-    ok = ok && eval(A, t, P, k3);
+    ok = ok && eval(A, t, P, k3, N);
     if (ok) jvp(A, t, P, dt_, d3);
 #pragma unroll
     for (int q = 0; q < 4; ++q) { t[q] = y[q] + k3[q] * A.dt; dt_[q] = dy[q] + d3[q] * A.dt; }
-    ok = ok && eval(A, t, P, k4);
+    ok = ok && eval(A, t, P, k4, N);
     if (ok) {
       jvp(A, t, P, dt_, d4);
 #pragma unroll
@@ -114,10 +116,13 @@ __global__ void __launch_bounds__(64) diff_tangent_kernel(DiffArgs<T> A) {
   A.status[i] = ok ? 0 : 1;
 }
 
-// FP32: capped at 96 registers (10 blocks of 64 per SM; measured fastest of
-// 8 / 10 / 12); FP64 uses what it needs (242).
+// The stages run in rolled loops (unrolled, instruction fetch was the bound:
+// 7.8 ms against 7.0 for 131,071 rays x 300 steps in FP32), each reading the
+// next one's state ahead.  FP32: 128 registers, 8 blocks of 64 per SM (7 blocks
+// 7.2 ms, 9 8.7, 10 9.4: what does not fit is spilled); 3,100 instructions a
+// warp-step at 59% of the issue slots bound it.  FP64 takes what it needs.
 template <typename T>
-__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 10 : 1) diff_adjoint_kernel(DiffArgs<T> A) {
+__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 1) diff_adjoint_kernel(DiffArgs<T> A) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= A.n) return;
   if (A.status[i] != 0) {  // no gradient through a ray that stopped
@@ -132,7 +137,8 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 10 : 1) diff_adjoint_kern
   acc.bkey = acc.ckey = -1;
 #pragma unroll
   for (int q = 0; q < 4; ++q) acc.d[q] = acc.u[q] = acc.v[q] = T(0);
-  const T half = A.dt * T(0.5), h = A.dt, sixth = A.dt / T(6);
+  Held<T> N;
+  const T half = A.dt * T(0.5), h = A.dt, sixth = A.dt / T(6), third = A.dt / T(3);
   for (int64_t seg = A.n_ck - 1; seg >= 0; --seg) {
     const int64_t first = seg * A.ck_every;
     const int64_t last = min(first + A.ck_every, A.steps);  // steps [first, last)
@@ -142,64 +148,69 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 10 : 1) diff_adjoint_kern
 #pragma unroll
     for (int q = 0; q < 4; ++q) y[q] = A.ckpt[(seg * 4 + q) * A.n + i];
     for (int64_t s = first; s < last; ++s) {
-      Point<T> P;
-      T k1[4], k2[4], k3[4], k4[4], Y2[4], Y3[4], Y4[4];
-      eval(A, y, P, k1);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) Y2[q] = y[q] + k1[q] * half;
-      eval(A, Y2, P, k2);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) Y3[q] = y[q] + k2[q] * half;
-      eval(A, Y3, P, k3);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) Y4[q] = y[q] + k3[q] * h;
       T *row = A.seg + (s - first) * 16 * A.n + i;
+      T Y[4], sum[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        row[q * A.n] = y[q];
-        row[(4 + q) * A.n] = Y2[q];
-        row[(8 + q) * A.n] = Y3[q];
-        row[(12 + q) * A.n] = Y4[q];
-      }
-      if (s + 1 < last) {
-        eval(A, Y4, P, k4);
+      for (int q = 0; q < 4; ++q) Y[q] = y[q];
+#pragma unroll 1
+      for (int st = 0; st < 4; ++st) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          y[q] = y[q] + (((k1[q] + k2[q] * T(2)) + k3[q] * T(2)) + k4[q]) * sixth;
+        for (int q = 0; q < 4; ++q) row[(4 * st + q) * A.n] = Y[q];
+        if (st == 3 && s + 1 == last) break;  // the last step's end is not needed
+        Point<T> P;
+        T k[4];
+        eval(A, Y, P, k, N);
+        const T wt = st == 0 || st == 3 ? T(1) : T(2), f = st == 2 ? h : half;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          sum[q] = sum[q] + k[q] * wt;
+          Y[q] = y[q] + k[q] * f;
+        }
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = y[q] + sum[q] * sixth;
     }
     // walk it backward: each stage's partials are evaluated where its
     // transpose is applied (one live Point)
+    T Yn[4];  // the next stage state, read ahead
     for (int64_t s = last - 1; s >= first; --s) {
       const T *row = A.seg + (s - first) * 16 * A.n + i;
-      Point<T> P;
-      T Ys[4], kd[4], w[4], r4[4], r3[4], r2[4], r1[4];
+      T r[4], r4[4], r3[4], r2[4];
+#pragma unroll 1
+      for (int st = 3; st >= 0; --st) {
+        Point<T> P;
+        T kd[4], w[4], Y[4];
+        if (st == 3 && s == last - 1) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) Ys[q] = row[(12 + q) * A.n];
-      eval(A, Ys, P, kd);
+          for (int q = 0; q < 4; ++q) Y[q] = row[(12 + q) * A.n];
+        } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = lam[q] * (h / T(6));
-      vjp(A, Ys, P, w, r4, acc);
+          for (int q = 0; q < 4; ++q) Y[q] = Yn[q];
+        }
+        if (st > 0 || s > first) {
+          const T *ahead = row + 4 * (st - 1) * A.n;  // of the step before for st = 0
 #pragma unroll
-      for (int q = 0; q < 4; ++q) Ys[q] = row[(8 + q) * A.n];
-      eval(A, Ys, P, kd);
+          for (int q = 0; q < 4; ++q) Yn[q] = ahead[q * A.n];
+        }
+        eval(A, Y, P, kd, N);
+        const T c = st == 3 || st == 0 ? sixth : third, f = st == 2 ? h : half;
+        if (st == 3) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = lam[q] * (h / T(3)) + h * r4[q];
-      vjp(A, Ys, P, w, r3, acc);
+          for (int q = 0; q < 4; ++q) w[q] = lam[q] * c;
+        } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) Ys[q] = row[(4 + q) * A.n];
-      eval(A, Ys, P, kd);
+          for (int q = 0; q < 4; ++q) w[q] = lam[q] * c + f * r[q];
+        }
+        vjp(A, Y, P, w, r, acc);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = lam[q] * (h / T(3)) + half * r3[q];
-      vjp(A, Ys, P, w, r2, acc);
+        for (int q = 0; q < 4; ++q) {
+          if (st == 3) r4[q] = r[q];
+          if (st == 2) r3[q] = r[q];
+          if (st == 1) r2[q] = r[q];
+        }
+      }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) Ys[q] = row[q * A.n];
-      eval(A, Ys, P, kd);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = lam[q] * (h / T(6)) + half * r2[q];
-      vjp(A, Ys, P, w, r1, acc);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) lam[q] = lam[q] + r1[q] + r2[q] + r3[q] + r4[q];
+      for (int q = 0; q < 4; ++q) lam[q] = lam[q] + r[q] + r2[q] + r3[q] + r4[q];
     }
   }
   flush_bathy(A, acc);

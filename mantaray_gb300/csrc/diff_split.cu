@@ -458,7 +458,8 @@ __device__ __forceinline__ bool forward_step(const SplitArgs &S, DiffCell &C, co
 
 __device__ __noinline__ bool fp64_rk4(const DiffArgs<double> &A, double *y) {
   double s[4] = {y[0], y[1], y[2], y[3]};
-  if (!rk4(A, s)) return false;
+  Held<double> N;
+  if (!rk4(A, s, N)) return false;
 #pragma unroll
   for (int q = 0; q < 4; ++q) y[q] = s[q];
   return true;
