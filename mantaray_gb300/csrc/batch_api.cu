@@ -539,8 +539,8 @@ int mr_batch_graph_create(mr_batch *b, size_t n_max, const uint8_t *ray_scenario
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   // the integrator build for this shape, chosen (an occupancy query) before
   // the capture begins
-  const void *k2 = mr::rk4_f32_function(cfg->rays_per_lane, cfg->block, cfg->blocks_per_sm,
-                                        batch_mode(b), cfg->staging,
+  const void *k2 = mr::rk4_f32_function(a.n, cfg->rays_per_lane, cfg->block,
+                                        cfg->blocks_per_sm, batch_mode(b), cfg->staging,
                                         gr->sweep);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {

@@ -43,10 +43,10 @@ cudaError_t launch_pack_bathy(const BathyDev &b, float4 *cells, cudaStream_t str
 cudaError_t launch_pack_current(const CurrentDev &c, float4 *cells, cudaStream_t stream);
 cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int rays_per_lane,
                            cudaStream_t stream);
-// The integrator build a launch of this shape runs in a mode (batch_mode;
+// The integrator build a launch of n rays and this shape runs in a mode (batch_mode;
 // staging: MR_STAGING_*; sweep: the sweep form; null where that build does
 // not exist); a graph's kernel node is found by it.
-const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int mode,
+const void *rk4_f32_function(int64_t n, int rays_per_lane, int block, int blocks_per_sm, int mode,
                              int staging, int sweep);
 // Dynamic shared memory of the tile build for blocks of `block` threads.
 size_t rk4_f32_tile_smem(int block);

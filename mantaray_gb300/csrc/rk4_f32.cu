@@ -6,7 +6,7 @@
 // K2 (rk4_f32_kernel_1 / _1r / _2, device code in k2.cuh): a persistent
 // kernel, grid = SMs x blocks per SM.  Each lane holds 1 or 2 rays (_2); one
 // ray per lane has an uncapped and a 64-register build (_1r), chosen by the
-// launch shape, and their sweep forms (_1s / _1rs: each launch advances its
+// launch shape and the number of rays, and their sweep forms (_1s / _1rs: each launch advances its
 // rays by at most sweep_steps steps, the rays still running re-sorted by
 // position between launches; batch_api.cu queues the sequence).  Each build
 // has two scenario-table forms (instantiated here) and two single-scenario
@@ -181,7 +181,7 @@ size_t rk4_f32_tile_smem(int block) {
   return static_cast<size_t>(block / 32) * (kTileBytes + 8);
 }
 
-const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, int mode,
+const void *rk4_f32_function(int64_t n, int rays_per_lane, int block, int blocks_per_sm, int mode,
                              int staging, int sweep) {
   if (mode == 4)  // results do not depend on the shape or the staging
     return sweep ? reinterpret_cast<const void *>(&rk4_f32_kernel_1s<4>)
@@ -219,7 +219,23 @@ const void *rk4_f32_function(int rays_per_lane, int block, int blocks_per_sm, in
       g_resident_1[sw][mode][slot].store(resident, std::memory_order_relaxed);
     }
   }
-  return resident < blocks_per_sm ? fn[1] : fn[0];
+  // The capped build for shapes beyond what the uncapped one keeps resident,
+  // unless all the call's rays fit in that: they then run at the latency of
+  // their own chain, which the cap's spills lengthen.  Blocks of 128, 12 per
+  // SM, 1,000 steps on 1,200^2 nodes, capped -> uncapped: seamount 10,000 rays
+  // 1,318 -> 1,161 us, 110,000 (the line is at 116,736) 1,872 -> 1,395; shelf
+  // 110,000 2,228 -> 1,644, in sweeps 2,848 -> 2,291.  Beyond the line either
+  // may win: 130,000 rays, seamount 1,879 -> 2,061, shelf 2,236 -> 1,769;
+  // 400,000, vortices in sweeps 5,838 -> 6,156, shelf 4,813 -> 4,592.
+  int dev = 0, sms = 0;
+  if (resident < blocks_per_sm &&
+      (cudaGetDevice(&dev) != cudaSuccess ||
+       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) {
+    (void)cudaGetLastError();
+    sms = 0;
+  }
+  return resident < blocks_per_sm && n > static_cast<int64_t>(sms) * resident * block ? fn[1]
+                                                                                      : fn[0];
 }
 
 cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int rays_per_lane,
@@ -231,7 +247,7 @@ cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>(sms * blocks_per_sm);
   void *args[] = {const_cast<BatchArgs *>(&a)};
-  const void *fn = rk4_f32_function(rays_per_lane, block, blocks_per_sm, a.mode, a.staging,
+  const void *fn = rk4_f32_function(a.n, rays_per_lane, block, blocks_per_sm, a.mode, a.staging,
                                     a.sweep_steps > 0);
   if (!fn) return cudaErrorInvalidValue;
   const size_t smem = a.mode == 4 ? 0
