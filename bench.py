@@ -43,7 +43,8 @@ GRID_BYTES_PER_RAY_STEP = 4 * 3 * 4 * 8
 OUT_BYTES_PER_ROW = 5 * 8
 # FP32 floating-point operations one ray-step of the batched kernel executes
 # (FADD/FMUL = 1, FFMA = 2), counted by ncu on the 4,096^2 shelf-slope case
-# with the current on the bathymetry's grid (92.0 FFMA, 36.0 FADD, 36.1 FMUL).
+# with the current on the bathymetry's grid (92.0 FFMA, 36.0 FADD, 36.1 FMUL),
+# before most of them moved to packed instructions, two to one (packed.cuh).
 FP32_FLOP_PER_RAY_STEP = 256.2
 # Algorithmic work of one ray-step (the reference's arithmetic, hand count from
 # src/wave_ray_path.rs:118-216 plus the RK4 update): ~55 FP64 add/mul/div per
@@ -54,15 +55,16 @@ FP32_FLOP_PER_RAY_STEP = 256.2
 ALG_FP64_FLOP_PER_RAY_STEP = 270.0
 ALG_FP32_FLOP_PER_RAY_STEP = 710.0
 # FP64 floating-point operations one ray-step executes (DADD/DMUL = 1,
-# DFMA = 2), per right-hand-side arithmetic, counted by ncu on the plain
-# kernel over the seamount workload's whole 4,000-step horizon (20,480 of its
+# DFMA = 2), per right-hand-side arithmetic, counted by ncu on the kernel that
+# the seamount runs (identity: the float-pair one, rk4_f64_grid.cu) over the seamount workload's whole 4,000-step horizon (20,480 of its
 # rays, 79.3 M ray-steps; sm__sass_thread_inst_executed_op_d{add,mul,fma}_pred_on).
-FP64_FLOP_PER_RAY_STEP = {"libm": 1399.1, "identity": 221.9}
+FP64_FLOP_PER_RAY_STEP = {"libm": 1399.1, "identity": 32.4}
 # FP64-pipe instructions per ray-step (sm__inst_executed_pipe_fp64 x 32: warp
 # instructions in lane slots, so lanes idle in a divergent warp count; same
-# captures), of the build the 65,536-ray benchmark runs: identity with the
-# lookup cache, libm without (its cached build does not fit one wave)
-FP64_PIPE_INST_PER_RAY_STEP = {"libm": 974.4, "identity": 225.4}
+# captures)
+FP64_PIPE_INST_PER_RAY_STEP = {"libm": 974.4, "identity": 30.2}
+# All instructions in lane slots (smsp__inst_executed x 32, same capture)
+INST_PER_RAY_STEP = {"identity": 1869.0}
 # DRAM bytes (read + written) per stored trajectory row of the plain kernel
 # on the seamount workload: ncu dram__bytes_read.sum + dram__bytes_write.sum
 # of one launch over its 65,536 rays x 1,000 steps (55.5 MB read, 2,573.7 MB
@@ -448,7 +450,10 @@ def gb300_arm(args, rank: int, world: int, local_rank: int):
         pass
     hbm_peak = peaks.get("hbm_gbs", 6800.0)
     # achieved = the algorithmic FP64 work of a ray-step (ALG_FP64_FLOP_PER_RAY_STEP)
-    # x ray-steps per second of the kernel; the executed work (ncu) beside it
+    # x ray-steps per second of the kernel; the executed work (ncu) beside it.
+    # The identity arithmetic does most of that work on pairs of floats, so its
+    # roofline is what it executes on the FP64 pipe, with the algorithmic figure
+    # (which passes the FP64 peak) and the issue slots beside it.
     fp64_achieved = rs_per_s_kernel * ALG_FP64_FLOP_PER_RAY_STEP / 1e12
     exec_flop = FP64_FLOP_PER_RAY_STEP[args.math]
     roofline = {"bound": "fp64", "achieved": fp64_achieved, "peak": fp64_peak.value,
@@ -464,6 +469,20 @@ def gb300_arm(args, rank: int, world: int, local_rank: int):
                 / (fp64_peak.value * 1e12 / 2.0),
                 "pipe_issue_note": "FP64-pipe instructions/s (ncu count per ray-step) over the "
                                    "FMA-chain DFMA/s"}
+    if args.math == "identity":
+        slots = rs_per_s_kernel * FP64_PIPE_INST_PER_RAY_STEP["identity"] / 1e12
+        props = torch.cuda.get_device_properties(dev)
+        roofline["algorithmic"] = {"achieved": fp64_achieved, "unit": "TFLOP/s",
+                                   "over_fp64_peak": fp64_achieved / fp64_peak.value,
+                                   "note": "the reference's FP64 operations, done on float pairs"}
+        roofline.update(achieved=slots, peak=fp64_peak.value / 2.0,
+                        unit="T FP64-pipe lane instructions/s",
+                        frac=2.0 * slots / fp64_peak.value,
+                        issue_slots_per_ray_step=INST_PER_RAY_STEP["identity"] / 32.0,
+                        issue_slots=rs_per_s_kernel * INST_PER_RAY_STEP["identity"] / 32.0
+                        / props.multi_processor_count)
+        roofline["issue_note"] = ("issue_slots: warp instructions per second and SM (ncu count per "
+                                  "ray-step); an SM issues 4 a clock")
     roofline["hbm"] = {"achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                        "frac": hbm_achieved / hbm_peak,
                        "bytes_per_ray_step": GRID_BYTES_PER_RAY_STEP + OUT_BYTES_PER_ROW,
