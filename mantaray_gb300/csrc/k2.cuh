@@ -22,6 +22,7 @@ namespace {
 // ------------------------------------------------------------------ K2 --
 
 constexpr int kCappedRegs = 64;  // of the capped builds (below)
+constexpr int kMiddleRegs = 72;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kGf = 9.8f;
 
@@ -898,8 +899,10 @@ __device__ __forceinline__ void k2_body(const BatchArgs &a) {
 // rays 14.8 / 14.5 / 14.1 / 15.6 ms.  With fewer rays than lanes the spills
 // only add latency.  Moving the origin, compensations and ray index to shared
 // memory instead (no spills at 64) gave 44.2 and 15.5 ms: not kept.
-// The launcher takes the capped build when the launch asks for more blocks
-// per SM than the uncapped one holds.
+// rk4_f32_kernel_1m is capped at 72 (28 warps): for the calls whose rays it
+// holds and the uncapped build does not, and in place of the 64-register sweep
+// form where the scenarios come from the table (more spills there).
+// rk4_f32_function has the rule.
 // Each comes in modes: 0 reads the lane's scenario from the device
 // table; 1 (one scenario) takes the scenario's fields from the kernel's
 // parameters (operands of the instructions instead of loads at every
@@ -913,7 +916,9 @@ template <int MODE>
 __global__ void __launch_bounds__(256) rk4_f32_kernel_1(BatchArgs a) { k2_body<1, MODE, 0>(a); }
 template <int MODE>
 __global__ void __maxnreg__(kCappedRegs) rk4_f32_kernel_1r(BatchArgs a) { k2_body<1, MODE, 0>(a); }
-// The sweep form of both: each launch advances its rays by at most
+template <int MODE>
+__global__ void __maxnreg__(kMiddleRegs) rk4_f32_kernel_1m(BatchArgs a) { k2_body<1, MODE, 0>(a); }
+// Their sweep forms: each launch advances its rays by at most
 // sweep_steps steps, the first from their initial states (sweep_first), the
 // later ones from the states the previous launch left.
 template <int MODE>
@@ -922,6 +927,8 @@ __global__ void __launch_bounds__(256) rk4_f32_kernel_1s(BatchArgs a) {
 }
 template <int MODE>
 __global__ void __maxnreg__(kCappedRegs) rk4_f32_kernel_1rs(BatchArgs a) { k2_body<1, MODE, 0, true>(a); }
+template <int MODE>
+__global__ void __maxnreg__(kMiddleRegs) rk4_f32_kernel_1ms(BatchArgs a) { k2_body<1, MODE, 0, true>(a); }
 // Two rays per lane hold twice the lane state: no cap.
 template <int MODE>
 __global__ void __launch_bounds__(256) rk4_f32_kernel_2(BatchArgs a) { k2_body<2, MODE, 0>(a); }

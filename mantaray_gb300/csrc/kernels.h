@@ -53,7 +53,7 @@ size_t rk4_f32_tile_smem(int block);
 // The single-scenario builds (rk4_f32_one.cu): 0 one ray per lane, 1 the same
 // capped (kCappedRegs), 2 two rays per lane, 3 the tile build, 4 the ahead
 // build (3 and 4: same grid only, else null), 5 and 6 the sweep form of 0
-// and 1.
+// and 1, 7 and 8 the middle build (kMiddleRegs) and its sweep form.
 const void *rk4_f32_one_function(int build, int same_grid);
 cudaError_t launch_fill_nan(float *p, int64_t count, cudaStream_t stream);
 

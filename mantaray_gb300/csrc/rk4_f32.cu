@@ -5,9 +5,10 @@
 //
 // K2 (rk4_f32_kernel_1 / _1r / _2, device code in k2.cuh): a persistent
 // kernel, grid = SMs x blocks per SM.  Each lane holds 1 or 2 rays (_2); one
-// ray per lane has an uncapped and a 64-register build (_1r), chosen by the
-// launch shape and the number of rays, and their sweep forms (_1s / _1rs: each launch advances its
-// rays by at most sweep_steps steps, the rays still running re-sorted by
+// ray per lane has an uncapped build and builds of 72 and 64 registers (_1m,
+// _1r), chosen by the launch shape and the number of rays, and their sweep
+// forms (_1s / _1ms / _1rs: each launch advances its rays by at most
+// sweep_steps steps, the rays still running re-sorted by
 // position between launches; batch_api.cu queues the sequence).  Each build
 // has two scenario-table forms (instantiated here) and two single-scenario
 // forms (rk4_f32_one.cu).  A lane whose ray has ended
@@ -46,6 +47,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "batch.h"
@@ -160,22 +162,35 @@ cudaError_t launch_fill_nan(float *p, int64_t count, cudaStream_t stream) {
 }
 
 // The builds of a table mode: [0] one ray per lane, uncapped; [1] the same
-// capped at kCappedRegs registers; [2] two rays per lane; [3] and [4] the sweep form of
-// [0] and [1].
+// capped at kCappedRegs registers; [2] two rays per lane; [3] the sweep form
+// of [0]; [4] the middle build (kMiddleRegs) and [5] its sweep form.
 template <int MODE>
 static const void *table_build(int k) {
-  static const void *builds[5] = {reinterpret_cast<const void *>(&rk4_f32_kernel_1<MODE>),
+  static const void *builds[6] = {reinterpret_cast<const void *>(&rk4_f32_kernel_1<MODE>),
                                   reinterpret_cast<const void *>(&rk4_f32_kernel_1r<MODE>),
                                   reinterpret_cast<const void *>(&rk4_f32_kernel_2<MODE>),
                                   reinterpret_cast<const void *>(&rk4_f32_kernel_1s<MODE>),
-                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1rs<MODE>)};
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1m<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1ms<MODE>)};
   return builds[k];
 }
 
-// Resident blocks per SM of each mode's uncapped one-ray build (plain and
-// sweep form) by block size (multiples of 32 up to 256), queried once; 0:
-// not yet known.
-static std::atomic<int> g_resident_1[2][6][9];
+// Resident blocks per SM of each mode's uncapped [0] and middle [1] one-ray
+// builds (plain and sweep form) by block size (multiples of 32 up to 256),
+// queried once; 0: not yet known.
+static std::atomic<int> g_resident[2][2][6][9];
+
+static int resident_blocks(const void *fn, int middle, int sweep, int mode, int block) {
+  const int slot = (block >= 32 && block <= 256 && block % 32 == 0) ? block / 32 : 0;
+  int r = slot ? g_resident[middle][sweep][mode][slot].load(std::memory_order_relaxed) : 0;
+  if (r != 0) return r;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, block, 0) != cudaSuccess || r < 1) {
+    (void)cudaGetLastError();
+    return 0;  // unknown
+  }
+  if (slot) g_resident[middle][sweep][mode][slot].store(r, std::memory_order_relaxed);
+  return r;
+}
 
 size_t rk4_f32_tile_smem(int block) {
   return static_cast<size_t>(block / 32) * (kTileBytes + 8);
@@ -195,47 +210,44 @@ const void *rk4_f32_function(int64_t n, int rays_per_lane, int block, int blocks
     if (mode == 5) return reinterpret_cast<const void *>(&rk4_f32_kernel_1a<5>);
     return nullptr;
   }
-  // [0] uncapped, [1] capped, [2] two rays per lane; the sweep form of [0]
-  // and [1] in their place
-  static const int kOneBuild[2][3] = {{0, 1, 2}, {5, 6, 2}};
-  static const int kTableBuild[2][3] = {{0, 1, 2}, {3, 4, 2}};
+  // [0] uncapped, [1] capped, [2] two rays per lane, [3] middle; their sweep
+  // forms in their place
+  static const int kOneBuild[2][4] = {{0, 1, 2, 7}, {5, 6, 2, 8}};
+  static const int kTableBuild[2][4] = {{0, 1, 2, 4}, {3, 5, 2, 5}};
   const int sw = sweep ? 1 : 0;
-  const void *fn[3];
-  for (int k = 0; k < 3; ++k)
+  const void *fn[4];
+  for (int k = 0; k < 4; ++k)
     fn[k] = mode == 1 || mode == 2 ? rk4_f32_one_function(kOneBuild[sw][k], mode == 2)
              : mode == 5            ? table_build<5>(kTableBuild[sw][k])
              : mode == 3            ? table_build<3>(kTableBuild[sw][k])
                                     : table_build<0>(kTableBuild[sw][k]);
   if (rays_per_lane == 2) return fn[2];
-  const int slot = (block >= 32 && block <= 256 && block % 32 == 0) ? block / 32 : 0;
-  int resident = slot ? g_resident_1[sw][mode][slot].load(std::memory_order_relaxed) : 0;
-  if (resident == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fn[0], block, 0) !=
-            cudaSuccess ||
-        resident < 1) {
-      (void)cudaGetLastError();
-      resident = blocks_per_sm;  // unknown: the uncapped build
-    } else if (slot) {
-      g_resident_1[sw][mode][slot].store(resident, std::memory_order_relaxed);
-    }
-  }
-  // The capped build for shapes beyond what the uncapped one keeps resident,
-  // unless all the call's rays fit in that: they then run at the latency of
-  // their own chain, which the cap's spills lengthen.  Blocks of 128, 12 per
-  // SM, 1,000 steps on 1,200^2 nodes, capped -> uncapped: seamount 10,000 rays
-  // 1,318 -> 1,161 us, 110,000 (the line is at 116,736) 1,872 -> 1,395; shelf
-  // 110,000 2,228 -> 1,644, in sweeps 2,848 -> 2,291.  Beyond the line either
-  // may win: 130,000 rays, seamount 1,879 -> 2,061, shelf 2,236 -> 1,769;
-  // 400,000, vortices in sweeps 5,838 -> 6,156, shelf 4,813 -> 4,592.
+  const int free_blocks = resident_blocks(fn[0], 0, sw, mode, block);
+  if (free_blocks == 0 || free_blocks >= blocks_per_sm) return fn[0];
+  // A launch that asks for more blocks per SM than the uncapped build keeps
+  // resident: the build with the most registers that holds all the call's
+  // rays at once, as they then run at the latency of their own chain, which a
+  // cap's spills lengthen; the capped one when none does.  Blocks of 128, 12
+  // per SM, 1,000 steps on 1,200^2 nodes, capped -> uncapped: seamount 10,000
+  // rays 1,318 -> 1,161 us, 110,000 (the line is at 116,736) 1,872 -> 1,395;
+  // shelf 110,000 2,228 -> 1,644, in sweeps 2,848 -> 2,291.  At 130,000 rays,
+  // capped / middle (to 136,192) / uncapped: two scenarios' seamount 1,912 /
+  // 1,681 us, one's in sweeps 2,574 / 2,388 / 2,919, the shelf's 2,939 / 2,676
+  // / 2,471.  Beyond, 400,000 rays: capped / middle, seamount of two scenarios
+  // 4,404 / 4,703, one in sweeps 5,061 / 5,202, but two in sweeps 5,552 /
+  // 5,529 and 1,200,000 13,743 / 13,205: the table's sweeps keep the middle
+  // one.
   int dev = 0, sms = 0;
-  if (resident < blocks_per_sm &&
-      (cudaGetDevice(&dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) {
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     (void)cudaGetLastError();
-    sms = 0;
+    return fn[1];
   }
-  return resident < blocks_per_sm && n > static_cast<int64_t>(sms) * resident * block ? fn[1]
-                                                                                      : fn[0];
+  auto holds = [&](int blocks) {
+    return n <= static_cast<int64_t>(sms) * std::min(blocks, blocks_per_sm) * block;
+  };
+  if (holds(free_blocks)) return fn[0];
+  return holds(resident_blocks(fn[3], 1, sw, mode, block)) ? fn[3] : fn[1];
 }
 
 cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int rays_per_lane,

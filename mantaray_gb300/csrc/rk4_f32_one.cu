@@ -22,6 +22,8 @@ static const void *one_build(int build) {
     case 1: return reinterpret_cast<const void *>(&rk4_f32_kernel_1r<MODE>);
     case 5: return reinterpret_cast<const void *>(&rk4_f32_kernel_1s<MODE>);
     case 6: return reinterpret_cast<const void *>(&rk4_f32_kernel_1rs<MODE>);
+    case 7: return reinterpret_cast<const void *>(&rk4_f32_kernel_1m<MODE>);
+    case 8: return reinterpret_cast<const void *>(&rk4_f32_kernel_1ms<MODE>);
     default: return reinterpret_cast<const void *>(&rk4_f32_kernel_2<MODE>);
   }
 }

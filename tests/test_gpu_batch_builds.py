@@ -1,6 +1,6 @@
-"""The batched kernel's capped build, taken when a call has more rays than the
-uncapped one keeps resident, against the uncapped build on a call that fits:
-the same rays, bit for bit, in both launch forms and table modes."""
+"""The batched kernel's capped and middle builds, taken when a call has more
+rays than the uncapped one keeps resident, against the uncapped build on a call
+that fits: the same rays, bit for bit, in both launch forms and table modes."""
 
 import numpy as np
 import pytest
@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("sweep", [0, 16])
 @pytest.mark.parametrize("scenarios", [1, 2])
-def test_capped_build_agrees(sweep, scenarios):
+@pytest.mark.parametrize("lanes", [7 * 128, 7 * 128 + 1, 2048])
+def test_capped_builds_agree(sweep, scenarios, lanes):
     import torch
 
     import mantaray_gb300 as mr
@@ -23,8 +24,9 @@ def test_capped_build_agrees(sweep, scenarios):
                mr.Current.grid(ax, ax, rng.normal(0, 0.2, (61, 61)),
                                rng.normal(0, 0.2, (61, 61)))) for _ in range(scenarios)]
     few = 4099
-    # beyond any residency: an SM holds 2,048 threads
-    many = 2048 * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    # per SM: what 72 registers hold (7 blocks of 128), one more, and beyond any
+    # residency
+    many = lanes * torch.cuda.get_device_properties(0).multi_processor_count
     th, k = rng.uniform(0, 2 * np.pi, few), rng.uniform(0.03, 0.3, few)
     rays = [rng.uniform(100, 1100, few), rng.uniform(100, 1100, few), k * np.cos(th),
             k * np.sin(th)]
