@@ -26,8 +26,10 @@
 // is the latency of dependent FP32 operations (2.3 of 4.6 cycles an
 // instruction), and the lanes of a warp in deep and in shallower water (22.5 of
 // 32 active).  The variant with FP64 equations in the reverse pass took 17.8 ms.
-// Tangent-linear, 8,192 rays x 500 steps: 16.2 ms in FP64, 5.3 here, one warp a
-// scheduler.
+// Tangent-linear, 8,192 rays x 500 steps: 16.2 ms in FP64, 5.8 here, one warp a
+// scheduler (5.5 with one unit for the call, which lost the tangents of every
+// ray far below the call's largest); along a depth tangent alone 5.8 (29.6:
+// lanes parted by steps in FP64 stayed parted).
 // Error against 128-bit arithmetic over 50 to 400 steps of 1 to 4 s on 200 to
 // 600 nodes a side, norm over norm, as a fraction of the FP64 kernels' error
 // (geometric mean of 8 cases): end positions and wavenumbers 0.97, gradients
@@ -85,43 +87,38 @@ struct SplitArgs {
   F2 dt2, half2, sixth2;
 };
 
-// Cell `cell`'s bilinear coefficients of nodes a, times u.
-__device__ __forceinline__ void coefficients(const double *a, int nx, int64_t cell, double u,
-                                             double o[4]) {
+// Cell `cell`'s bilinear coefficients of nodes a.
+__device__ __forceinline__ void coefficients(const double *a, int nx, int64_t cell, double o[4]) {
   const int64_t base = cell / (nx - 1) * nx + cell % (nx - 1);
-  const double v00 = u * a[base], v10 = u * a[base + 1], v01 = u * a[base + nx],
-               v11 = u * a[base + nx + 1];
+  const double v00 = a[base], v10 = a[base + 1], v01 = a[base + nx], v11 = a[base + nx + 1];
   o[0] = v00;
   o[1] = v10 - v00;
   o[2] = v01 - v00;
   o[3] = ((v11 - v10) - v01) + v00;
 }
 
-// A bathymetry's (current's) cell as pairs, and in FP64 where b64 (c64) is
-// given.  A null u or v counts as zero.
-__device__ __forceinline__ void bathy_record(const double *a, int nx, int64_t k, double unit,
-                                             float4 *b, double2 *b64) {
+// A bathymetry's (current's) cell as pairs and in FP64.
+__device__ __forceinline__ void bathy_record(const double *a, int nx, int64_t k, float4 *b,
+                                             double2 *b64) {
   double o[4];
-  coefficients(a, nx, k, unit, o);
+  coefficients(a, nx, k, o);
   F2 q[4];
   for (int t = 0; t < 4; ++t) q[t] = to_pair(o[t]);
   b[2 * k] = make_float4(q[0].h, q[1].h, q[2].h, q[3].h);
   b[2 * k + 1] = make_float4(q[0].l, q[1].l, q[2].l, q[3].l);
-  if (b64) {
-    b64[2 * k] = make_double2(o[0], o[1]);
-    b64[2 * k + 1] = make_double2(o[2], o[3]);
-  }
+  b64[2 * k] = make_double2(o[0], o[1]);
+  b64[2 * k + 1] = make_double2(o[2], o[3]);
 }
 __device__ __forceinline__ void current_record(const double *u, const double *v, int nx, int64_t k,
-                                               double unit, float4 *c, double2 *c64) {
-  double o[4] = {0.0, 0.0, 0.0, 0.0}, p[4] = {0.0, 0.0, 0.0, 0.0};
-  if (u) coefficients(u, nx, k, unit, o);
-  if (v) coefficients(v, nx, k, unit, p);
+                                               float4 *c, double2 *c64) {
+  double o[4], p[4];
+  coefficients(u, nx, k, o);
+  coefficients(v, nx, k, p);
   F2 q[4], r[4];
   for (int t = 0; t < 4; ++t) {
     q[t] = to_pair(o[t]);
     r[t] = to_pair(p[t]);
-    if (c64) c64[4 * k + t] = make_double2(o[t], p[t]);
+    c64[4 * k + t] = make_double2(o[t], p[t]);
   }
   c[4 * k] = make_float4(q[0].h, r[0].h, q[1].h, r[1].h);
   c[4 * k + 1] = make_float4(q[2].h, r[2].h, q[3].h, r[3].h);
@@ -132,9 +129,9 @@ __device__ __forceinline__ void current_record(const double *u, const double *v,
 __global__ void build_diff_records(SplitArgs S, float4 *b, double2 *b64, float4 *c, double2 *c64) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k < static_cast<int64_t>(S.b.nx - 1) * (S.b.ny - 1))
-    bathy_record(S.A.bg.a, S.b.nx, k, 1.0, b, b64);
+    bathy_record(S.A.bg.a, S.b.nx, k, b, b64);
   if (k < static_cast<int64_t>(S.c.nx - 1) * (S.c.ny - 1))
-    current_record(S.A.cg.a, S.A.cg.b, S.c.nx, k, 1.0, c, c64);
+    current_record(S.A.cg.a, S.A.cg.b, S.c.nx, k, c, c64);
 }
 
 // The cells a lane holds.
@@ -502,7 +499,7 @@ __global__ void __launch_bounds__(kSplitBlock, 6)
 
 // ---------------------------------------------------------------- adjoint --
 
-// The adjoint (tangent) state is held in units of 2^e, e the exponent of its
+// The adjoint state is held in units of 2^e, e the exponent of its
 // largest component at the start (floats reach from 2^-126 to 2^128, gradients
 // can be anything); e = 0 when that is beyond 2^+-900.
 __device__ __forceinline__ uint32_t high_word(double v) {
@@ -880,49 +877,107 @@ __global__ void __launch_bounds__(kSplitBlock, 4)
 
 // ---------------------------------------------------------------- tangent --
 
-// The tangent form's own arguments: the tangent fields' records, in the call's
-// unit (null: none), and the high word of that unit, 0 where floats do not
-// hold the tangents (every step then runs in FP64).
+// The tangent form's own arguments: the tangent fields' records, as those of
+// the fields but each cell's (u's and v's apart) in units of 2^e, e the
+// exponent of its largest coefficient, and that exponent as in a double's high
+// word (0: all zero; kNoRecord: not finite, or beyond 2^+-850).  Null: none.
+//
+// Tangents have no natural size, and those of one call may span any range (a
+// fill value at a node no ray meets, one ray among many), so each step of each
+// ray has a unit too, a power of two near the largest component of its tangent
+// (while that is 0: its cells' largest coefficient), and the pairs hold values
+// in that unit.  A step is on pairs where, in units,
+//   each component of the ray's tangent is 0 or at least 2^-100 (below, its
+//   pair loses the low half), and
+//   each cell's largest coefficient is 0, or 2^-72 to 2^120 (what the smaller
+//   ones lose, 2^-124, is then below the rounding of the nodes' differences),
+//   or less where every component of the ray's tangent is 2^-30 or more (and
+//   that loss is below its rounding);
+// every other step, and one whose result is not finite, runs in FP64.
 struct TangentArgs {
   SplitArgs S;
   const float4 *db, *dc;
-  const uint32_t *unit;
+  const uint32_t *db_e;
+  const uint2 *dc_e;
+};
+constexpr uint32_t kNoRecord = 0x7ff00000u;
+
+// The cells of the tangent fields that a lane holds, in units; tiny: a
+// coefficient field is nonzero and below 2^-72 units, bad: not covered.
+struct TangentCell : DiffCell {
+  bool b_tiny = false, b_bad = false, c_tiny = false, c_bad = false;
 };
 
-// The largest high word of the tangents given.
-__global__ void largest_tangent(DiffArgs<double> A, uint32_t *word) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t bn = static_cast<int64_t>(A.bg.nx) * A.bg.ny;
-  const int64_t cn = static_cast<int64_t>(A.cg.nx) * A.cg.ny;
-  uint32_t w = 0;
-  for (int64_t k = t0; k < 4 * A.n; k += stride) w = max(w, high_word(A.dstate0[k]));
-  if (A.d_depth)
-    for (int64_t k = t0; k < bn; k += stride) w = max(w, high_word(A.d_depth[k]));
-  for (int64_t k = t0; k < cn; k += stride) {
-    if (A.d_u) w = max(w, high_word(A.d_u[k]));
-    if (A.d_v) w = max(w, high_word(A.d_v[k]));
-  }
-  w = __reduce_max_sync(0xffffffffu, w);
-  if ((threadIdx.x & 31) == 0 && w) atomicMax(word, w);
+// Order of magnitude: the high word, at least 1 for anything but 0.
+__device__ __forceinline__ uint32_t magnitude_word(double v) {
+  return high_word(v) | (static_cast<uint32_t>(bits_of(v)) != 0u ? 1u : 0u);
+}
+__device__ __forceinline__ uint32_t exponent_word(const double o[4]) {
+  const uint32_t w = max(max(magnitude_word(o[0]), magnitude_word(o[1])),
+                         max(magnitude_word(o[2]), magnitude_word(o[3])));
+  return w == 0 || (w >= (173u << 20) && w < (1873u << 20)) ? w & 0x7ff00000u : kNoRecord;
 }
 
-// The unit's high word from the largest one.
-__device__ __forceinline__ uint32_t tangent_unit(uint32_t word) {
-  const uint32_t e = word >> 20;
-  return word == 0 ? 1023u << 20 : e > 123 && e < 1923 ? e << 20 : 0u;
+// A unit is given as `sh`: its exponent, in place to be added to a high word.
+// v is below 2^127 units.  split3's parts, with a low half down to 2^-149.
+__device__ __forceinline__ F2 pair_in_units(double v, int32_t sh) {
+  const uint32_t hi = static_cast<uint32_t>(bits_of(v) >> 32), lo = static_cast<uint32_t>(bits_of(v));
+  const uint32_t sign = hi & 0x80000000u;
+  const int32_t e = static_cast<int32_t>((hi >> 20) & 0x7ffu) - (sh >> 20) - 1023;
+  const float h = float_of(sign | static_cast<uint32_t>(e + 127) << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
+  // the 29 bits after, in units of 2^(e - 52)
+  const uint32_t n = lo & 0x1fffffffu;
+  const float t = fma32(float_of(0x4b000000u | n >> 6) - 8388608.0f, 64.0f,
+                        float_of(0x4b000000u | (n & 63u)) - 8388608.0f);
+  const float l = (t * 0x1p-26f) * float_of(sign | static_cast<uint32_t>(e - 26 + 127) << 23);
+  return F2{e < -126 ? 0.0f : h, e < -100 ? 0.0f : l};
+}
+__device__ __forceinline__ double from_units(float f, int32_t sh) {
+  if (f == 0.0f) return 0.0;
+  const uint64_t b = bits_of(f2d_normal(f));
+  return double_of(static_cast<uint32_t>(b >> 32) + static_cast<uint32_t>(sh),
+                   static_cast<uint32_t>(b));
+}
+// On the floats: their conversions to doubles make infinities and NaN finite.
+__device__ __forceinline__ bool all_finite(V2 a) {
+  const V s = vadd(a.h, a.l);
+  return fabsf(s.x) < 0x1p126f && fabsf(s.y) < 0x1p126f;
 }
 
-__global__ void build_tangent_records(TangentArgs T, float4 *db, float4 *dc) {
+__global__ void build_tangent_records(TangentArgs T, float4 *db, float4 *dc, uint32_t *db_e,
+                                      uint2 *dc_e) {
   const DiffArgs<double> &A = T.S.A;
-  const uint32_t unit = tangent_unit(*T.unit);
-  if (!unit) return;
-  const double per = double_of(0x7fe00000u - unit, 0u);
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (db && k < static_cast<int64_t>(A.bg.nx - 1) * (A.bg.ny - 1))
-    bathy_record(A.d_depth, A.bg.nx, k, per, db, nullptr);
-  if (dc && k < static_cast<int64_t>(A.cg.nx - 1) * (A.cg.ny - 1))
-    current_record(A.d_u, A.d_v, A.cg.nx, k, per, dc, nullptr);
+  auto unit = [](uint32_t w) {
+    return w == 0 || w == kNoRecord ? 0 : static_cast<int32_t>(w) - (1023 << 20);
+  };
+  if (db && k < static_cast<int64_t>(A.bg.nx - 1) * (A.bg.ny - 1)) {
+    double o[4];
+    F2 q[4];
+    coefficients(A.d_depth, A.bg.nx, k, o);
+    const uint32_t w = exponent_word(o);
+    db_e[k] = w;
+    for (int t = 0; t < 4; ++t)
+      q[t] = w == kNoRecord ? F2{0.0f, 0.0f} : pair_in_units(o[t], unit(w));
+    db[2 * k] = make_float4(q[0].h, q[1].h, q[2].h, q[3].h);
+    db[2 * k + 1] = make_float4(q[0].l, q[1].l, q[2].l, q[3].l);
+  }
+  if (dc && k < static_cast<int64_t>(A.cg.nx - 1) * (A.cg.ny - 1)) {
+    double o[4] = {0.0, 0.0, 0.0, 0.0}, p[4] = {0.0, 0.0, 0.0, 0.0};
+    F2 q[4], r[4];
+    if (A.d_u) coefficients(A.d_u, A.cg.nx, k, o);
+    if (A.d_v) coefficients(A.d_v, A.cg.nx, k, p);
+    const uint32_t wu = exponent_word(o), wv = exponent_word(p);
+    dc_e[k] = make_uint2(wu, wv);
+    for (int t = 0; t < 4; ++t) {
+      q[t] = wu == kNoRecord ? F2{0.0f, 0.0f} : pair_in_units(o[t], unit(wu));
+      r[t] = wv == kNoRecord ? F2{0.0f, 0.0f} : pair_in_units(p[t], unit(wv));
+    }
+    dc[4 * k] = make_float4(q[0].h, r[0].h, q[1].h, r[1].h);
+    dc[4 * k + 1] = make_float4(q[2].h, r[2].h, q[3].h, r[3].h);
+    dc[4 * k + 2] = make_float4(q[0].l, r[0].l, q[1].l, r[1].l);
+    dc[4 * k + 3] = make_float4(q[2].l, r[2].l, q[3].l, r[3].l);
+  }
 }
 
 // One stage's tangent of (dx, dk): m = M dk, t = m + the rest, and tk.
@@ -952,36 +1007,98 @@ __device__ __forceinline__ void stage_jvp(const SplitArgs &S, const DiffCell &C,
   *tk = sub(mul(g, S.b.inv), mul(lanes(tx, ty), S.c.inv));
 }
 
-// The tangent fields' cells of a stage, those the lane holds in C.
-__device__ __forceinline__ void take_tangent_cells(const TangentArgs &T, const DiffCell &C,
-                                                   DiffCell &D) {
+// A record's factor into units of sh, its exponent w (0 where that is below a
+// float's, which is used only where tiny is allowed).
+__device__ __forceinline__ float unit_factor(uint32_t w, int32_t sh, bool *tiny, bool *bad) {
+  const int32_t d = static_cast<int32_t>(w >> 20) - (sh >> 20) - 1023;
+  *bad |= d > 120;
+  *tiny |= w != 0 && d < -72;
+  return w == 0 || d < -126 || d > 120 ? 0.0f : float_of(static_cast<uint32_t>(d + 127) << 23);
+}
+__device__ __forceinline__ float4 scaled(float4 a, float f, float g) {  // lanes x, z and y, w
+  return make_float4(a.x * f, a.y * g, a.z * f, a.w * g);
+}
+
+// The tangent fields' cells of a stage, those the lane holds in C; false where
+// the pairs do not cover them.  full: every component of the ray's tangent is
+// 2^-30 units or more.
+__device__ __forceinline__ bool take_tangent_cells(const TangentArgs &T, const DiffCell &C,
+                                                   int32_t sh, bool full, TangentCell &D) {
   if (T.db && D.bkey != C.bkey) {
     const float4 *p = T.db + static_cast<int64_t>(C.bkey) * 2;
-    D.b[0] = ld4(p);
-    D.b[1] = ld4(p + 1);
+    D.b_tiny = D.b_bad = false;
+    const float f = unit_factor(__ldg(T.db_e + C.bkey), sh, &D.b_tiny, &D.b_bad);
+    D.b[0] = scaled(ld4(p), f, f);
+    D.b[1] = scaled(ld4(p + 1), f, f);
     D.bkey = C.bkey;
   }
   if (T.dc && D.ckey != C.ckey) {
     const float4 *p = T.dc + static_cast<int64_t>(C.ckey) * 4;
+    const uint2 w = __ldg(T.dc_e + C.ckey);
+    D.c_tiny = D.c_bad = false;
+    const float f = unit_factor(w.x, sh, &D.c_tiny, &D.c_bad);
+    const float g = unit_factor(w.y, sh, &D.c_tiny, &D.c_bad);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) D.c[q] = ld4(p + q);
+    for (int q = 0; q < 4; ++q) D.c[q] = scaled(ld4(p + q), f, g);
     D.ckey = C.ckey;
   }
+  return !(D.b_bad || D.c_bad) && (full || !(D.b_tiny || D.c_tiny));
+}
+
+// The unit of a step of tangent dy from the point b, c: the last step's while
+// it is within 2^30 of dy's largest component.  False where the pairs do not
+// cover dy.
+template <bool SAME>
+__device__ __forceinline__ bool choose_unit(const TangentArgs &T, const Base &b, const Base &c,
+                                            const double dy[4], int32_t *sh, bool *full,
+                                            TangentCell &D) {
+  uint32_t w[4], top = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    w[q] = magnitude_word(dy[q]);
+    top = max(top, w[q]);
+  }
+  if (top == 0) {
+    if (T.db) top = __ldg(T.db_e + (b.j * (T.S.b.nx - 1) + b.i));
+    if (T.dc) {
+      const Base &g = SAME ? b : c;
+      const uint2 e = __ldg(T.dc_e + (g.j * (T.S.c.nx - 1) + g.i));
+      top = max(top, max(e.x, e.y));
+    }
+    if (top == 0) top = 1023u << 20;  // nothing but zeros
+  }
+  if (top < (173u << 20) || top >= (1873u << 20)) return false;
+  const bool change = static_cast<int32_t>(top) < (993 << 20) + *sh ||
+                      static_cast<int32_t>(top) > (1053 << 20) + *sh;
+  *sh = change ? static_cast<int32_t>(top & 0x7ff00000u) - (1023 << 20) : *sh;
+  D.bkey = change ? -1 : D.bkey;
+  D.ckey = change ? -1 : D.ckey;
+  bool ok = true;
+  *full = true;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int32_t m = static_cast<int32_t>(w[q]) - *sh;
+    ok &= w[q] == 0 || m >= (923 << 20);
+    *full &= w[q] != 0 && m >= (993 << 20);
+  }
+  return ok;
 }
 
 // A step of the state and its tangent; false (y and dy as they were) when a
-// stage is outside the pairs' domain.
+// stage is outside the pairs' domain.  sh: the unit, kept from step to step.
 template <bool SAME>
-__device__ __forceinline__ bool tangent_step(const TangentArgs &T, DiffCell &C, DiffCell &D,
-                                             double y[4], double dy[4]) {
+__device__ __forceinline__ bool tangent_step(const TangentArgs &T, DiffCell &C, TangentCell &D,
+                                             int32_t &sh, double y[4], double dy[4]) {
   const SplitArgs &S = T.S;
   Base b, c;
   if (!base_of(S.b, y[0], y[1], &b)) return false;
   if (!SAME && !base_of(S.c, y[0], y[1], &c)) return false;
   const V2 k = lanes(to_pair(y[2]), to_pair(y[3]));
-  const V2 dx0 = lanes(to_pair(dy[0]), to_pair(dy[1]));
-  const V2 dk0 = lanes(to_pair(dy[2]), to_pair(dy[3]));
   const bool depth = T.db != nullptr, current = T.dc != nullptr;
+  bool full;
+  if (!choose_unit<SAME>(T, b, c, dy, &sh, &full, D)) return false;
+  const V2 dx0 = lanes(pair_in_units(dy[0], sh), pair_in_units(dy[1], sh));
+  const V2 dk0 = lanes(pair_in_units(dy[2], sh), pair_in_units(dy[3], sh));
   V2 disp = zero2(), q = k, dx = dx0, dq = dk0;       // the stage's state
   V2 d1 = disp, k1 = disp, m1 = disp, sd = disp, sk = disp, sdx = disp, sdk = disp;
   double a[4] = {0.0, 0.0, 0.0, 0.0}, mx = 0.0, my = 0.0;  // anchors
@@ -989,7 +1106,7 @@ __device__ __forceinline__ bool tangent_step(const TangentArgs &T, DiffCell &C, 
   for (int st = 0; st < 4; ++st) {
     At p;
     if (!stage_at<SAME>(S, b, c, disp, C, &p)) return false;
-    take_tangent_cells(T, C, D);
+    if (!take_tangent_cells(T, C, sh, full, D)) return false;
     const Wave wv = wave_of(q);
     if (!diff_ok(p, wv.k2.h)) return false;
     Eqs e;
@@ -1025,14 +1142,15 @@ __device__ __forceinline__ bool tangent_step(const TangentArgs &T, DiffCell &C, 
   }
   const V2 s6 = mul(sd, both(S.sixth2)), k6 = mul(sk, both(S.sixth2));
   const V2 t6 = mul(sdx, both(S.sixth2));
+  if (!(all_finite(t6) && all_finite(sdk))) return false;
   y[0] += fma(S.A.dt, a[0], f2d_zero(s6.h.x)) + f2d_zero(s6.l.x);
   y[1] += fma(S.A.dt, a[1], f2d_zero(s6.h.y)) + f2d_zero(s6.l.y);
   y[2] += fma(S.A.dt, a[2], f2d_zero(k6.h.x)) + f2d_zero(k6.l.x);
   y[3] += fma(S.A.dt, a[3], f2d_zero(k6.h.y)) + f2d_zero(k6.l.y);
-  dy[0] += fma(S.A.dt, mx, f2d_zero(t6.h.x)) + f2d_zero(t6.l.x);
-  dy[1] += fma(S.A.dt, my, f2d_zero(t6.h.y)) + f2d_zero(t6.l.y);
-  dy[2] = fma(S.sixth, to_double(x_of(sdk)), dy[2]);
-  dy[3] = fma(S.sixth, to_double(y_of(sdk)), dy[3]);
+  dy[0] += fma(S.A.dt, mx, from_units(t6.h.x, sh)) + from_units(t6.l.x, sh);
+  dy[1] += fma(S.A.dt, my, from_units(t6.h.y, sh)) + from_units(t6.l.y, sh);
+  dy[2] = fma(S.sixth, from_units(sdk.h.x, sh) + from_units(sdk.l.x, sh), dy[2]);
+  dy[3] = fma(S.sixth, from_units(sdk.h.y, sh) + from_units(sdk.l.y, sh), dy[3]);
   return true;
 }
 
@@ -1069,33 +1187,34 @@ __global__ void __launch_bounds__(kSplitBlock)
     diff_split_tangent(const __grid_constant__ TangentArgs T) {
   const DiffArgs<double> &A = T.S.A;
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned lanes_of_warp = __ballot_sync(0xffffffffu, i < A.n);
   if (i >= A.n) return;
   double y[4] = {A.x0[i], A.y0[i], A.kx0[i], A.ky0[i]};
-  const uint32_t word = tangent_unit(*T.unit);
-  const bool pairs = word != 0;
-  const double unit = pairs ? double_of(word, 0u) : 1.0;
-  const double per = pairs ? double_of(0x7fe00000u - word, 0u) : 1.0;
   double dy[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) dy[q] = A.dstate0[q * A.n + i] * per;
+  for (int q = 0; q < 4; ++q) dy[q] = A.dstate0[q * A.n + i];
   bool ok = true;
-  DiffCell C, D;
+  DiffCell C;
+  TangentCell D;
+  int32_t sh = 0;
   for (int64_t s = 0; s < A.steps; ++s) {
-    if (!(pairs && in_units(dy) && tangent_step<SAME>(T, C, D, y, dy))) {
+    if (ok && !tangent_step<SAME>(T, C, D, sh, y, dy)) {
       double yv[4], dv[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) { yv[q] = y[q]; dv[q] = dy[q] * unit; }
+      for (int q = 0; q < 4; ++q) { yv[q] = y[q]; dv[q] = dy[q]; }
       ok = fp64_tangent(A, yv, dv);
-      if (!ok) break;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) { y[q] = yv[q]; dy[q] = dv[q] * per; }
+      for (int q = 0; q < 4; ++q) { y[q] = yv[q]; dy[q] = dv[q]; }
     }
+    // Together again: lanes that a step has parted (a new unit, a step in FP64)
+    // otherwise stay so to the end, at twice the time.
+    if ((s & 7) == 7 && !__any_sync(lanes_of_warp, ok)) break;
   }
   const double nan = NAN;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     A.end_state[q * A.n + i] = ok ? y[q] : nan;
-    A.d_end[q * A.n + i] = ok ? dy[q] * unit : nan;
+    A.d_end[q * A.n + i] = ok ? dy[q] : nan;
   }
   A.status[i] = ok ? 0 : 1;
 }
@@ -1169,7 +1288,9 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   const size_t records = static_cast<size_t>(bn) * 64 + static_cast<size_t>(cn) * 128;
   const size_t db_bytes = db ? static_cast<size_t>(bn) * 32 : 0;
   const size_t dc_bytes = dc ? static_cast<size_t>(cn) * 64 : 0;
-  const size_t bytes = records + db_bytes + dc_bytes + 16;
+  const size_t dce_bytes = dc ? static_cast<size_t>(cn) * 8 : 0;
+  const size_t dbe_bytes = db ? static_cast<size_t>(bn) * 4 : 0;
+  const size_t bytes = records + db_bytes + dc_bytes + dce_bytes + dbe_bytes;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
       cudaMallocAsync(reinterpret_cast<void **>(&mem), bytes, stream) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -1195,15 +1316,15 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
     else
       diff_split_adjoint<false><<<grid, kSplitBlock, 0, stream>>>(S);
   } else {
-    uint32_t *unit = reinterpret_cast<uint32_t *>(mem + records + db_bytes + dc_bytes);
-    float4 *dbr = db ? reinterpret_cast<float4 *>(mem + records) : nullptr;
-    float4 *dcr = dc ? reinterpret_cast<float4 *>(mem + records + db_bytes) : nullptr;
-    const TangentArgs T{S, dbr, dcr, unit};
-    (void)cudaMemsetAsync(unit, 0, sizeof(uint32_t), stream);
-    largest_tangent<<<304, 256, 0, stream>>>(A, unit);
+    char *p = mem + records;
+    float4 *dbr = db ? reinterpret_cast<float4 *>(p) : nullptr;
+    float4 *dcr = dc ? reinterpret_cast<float4 *>(p += db_bytes) : nullptr;
+    uint2 *dce = dc ? reinterpret_cast<uint2 *>(p += dc_bytes) : nullptr;
+    uint32_t *dbe = db ? reinterpret_cast<uint32_t *>(mem + bytes - dbe_bytes) : nullptr;
+    const TangentArgs T{S, dbr, dcr, dbe, dce};
     if (db || dc)
-      build_tangent_records<<<static_cast<unsigned>((cells + 255) / 256), 256, 0, stream>>>(T, dbr,
-                                                                                            dcr);
+      build_tangent_records<<<static_cast<unsigned>((cells + 255) / 256), 256, 0, stream>>>(
+          T, dbr, dcr, dbe, dce);
     if (k.same_grid)
       diff_split_tangent<true><<<grid, kSplitBlock, 0, stream>>>(T);
     else
