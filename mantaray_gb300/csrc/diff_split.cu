@@ -56,6 +56,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+#include <vector>
+
 #define MR_SPLIT_LOW_PRODUCT
 #include "diff.cuh"
 #include "diff_split.h"
@@ -1239,6 +1242,27 @@ SplitField field_of(int nx, int ny, double x0, double y0, double inv_dx, double 
 
 bool in_range(double v) { return v > 0x1p-20 && v < 0x1p20; }
 
+// The pool the records come from, one per device for the process (null: none).
+// Apart from the device's default pool, which mr_trace has keep what is freed:
+// this one has the default release threshold of 0 and gives it back at the
+// stream's next synchronisation.
+cudaMemPool_t record_pool() {
+  static std::mutex mu;
+  static std::vector<cudaMemPool_t> pools;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (static_cast<size_t>(device) >= pools.size()) pools.resize(device + 1, nullptr);
+  if (!pools[device]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&pools[device], &props) != cudaSuccess) pools[device] = nullptr;
+  }
+  return pools[device];
+}
+
 }  // namespace
 
 bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cudaError_t *err) {
@@ -1278,9 +1302,7 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   S.sixth2 = host_pair(S.sixth);
   // Stream-ordered scratch for the records, freed behind the kernels; not
   // while the stream is being captured (the allocation would become a node of
-  // the caller's graph).  From the device's own pool, which gives it back at
-  // the next synchronisation: 0.2 ms a call for the 50 MB of 512 x 512 cells,
-  // where the kernels are 44 -> 14.2 ms.
+  // the caller's graph).
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   char *mem = nullptr;
   const bool db = form == DIFF_TANGENT && k.d_depth;
@@ -1291,8 +1313,11 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   const size_t dce_bytes = dc ? static_cast<size_t>(cn) * 8 : 0;
   const size_t dbe_bytes = db ? static_cast<size_t>(bn) * 4 : 0;
   const size_t bytes = records + db_bytes + dc_bytes + dce_bytes + dbe_bytes;
+  cudaMemPool_t pool = nullptr;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-      cudaMallocAsync(reinterpret_cast<void **>(&mem), bytes, stream) != cudaSuccess) {
+      !(pool = record_pool()) ||
+      cudaMallocFromPoolAsync(reinterpret_cast<void **>(&mem), bytes, pool, stream) !=
+          cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }

@@ -4,8 +4,6 @@ tangent among others', components and fields decades apart.  Against
 diff_reference.cpp, each ray's tangent over the ray's own scale, with the
 bound of test_gpu_diff_split.py (100 s 2^-45 in norm for s steps)."""
 
-import ctypes
-
 import numpy as np
 import pytest
 
