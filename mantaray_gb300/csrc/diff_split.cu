@@ -1244,8 +1244,11 @@ bool in_range(double v) { return v > 0x1p-20 && v < 0x1p20; }
 
 // The pool the records come from, one per device for the process (null: none).
 // Apart from the device's default pool, which mr_trace has keep what is freed:
-// this one has the default release threshold of 0 and gives it back at the
-// stream's next synchronisation.
+// this one keeps kKeptBytes at most and gives the rest back at the next
+// synchronisation.  Mapping memory anew takes a call some 140 us and 150 ps a
+// cell, as long as seven steps of few rays.  It does not make one stream wait
+// for another to reuse memory.
+constexpr uint64_t kKeptBytes = 64ull << 20;
 cudaMemPool_t record_pool() {
   static std::mutex mu;
   static std::vector<cudaMemPool_t> pools;
@@ -1258,7 +1261,17 @@ cudaMemPool_t record_pool() {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
-    if (cudaMemPoolCreate(&pools[device], &props) != cudaSuccess) pools[device] = nullptr;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kKeptBytes;
+    int no = 0;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no) !=
+            cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return nullptr;
+    }
+    pools[device] = pool;
   }
   return pools[device];
 }
@@ -1269,15 +1282,37 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   const int64_t bn = static_cast<int64_t>(k.bnx - 1) * (k.bny - 1);
   const int64_t cn = static_cast<int64_t>(k.cnx - 1) * (k.cny - 1);
   const int64_t cells = bn > cn ? bn : cn;
-  // The records cost about 40 ps a cell (192 bytes written, 24 read).  A
-  // ray-step on pairs saves over 1 ns of the FP64 kernels' time, and a step of
-  // however few rays over 5 us of their dependent chain (2^16 cells: 2.6 us).
-  // 217 rays x 79 steps, adjoint on 544^2 nodes: 5.8 -> 2.9 ms; 191 x 65,
-  // tangent on 476^2: 2.2 -> 0.9.
-  if (k.n == 0 || k.steps == 0 || k.n > (1ll << 40) / k.steps || cells > (16 * k.n + 65536) * k.steps ||
-      cells > (1ll << 26) || k.bnx > (1 << 20) || k.bny > (1 << 20) || k.cnx > (1 << 20) ||
-      k.cny > (1 << 20))
+  const bool db = form == DIFF_TANGENT && k.d_depth;
+  const bool dc = form == DIFF_TANGENT && (k.d_u || k.d_v);
+  const size_t records = static_cast<size_t>(bn) * 64 + static_cast<size_t>(cn) * 128;
+  const size_t db_bytes = db ? static_cast<size_t>(bn) * 32 : 0;
+  const size_t dc_bytes = dc ? static_cast<size_t>(cn) * 64 : 0;
+  const size_t dce_bytes = dc ? static_cast<size_t>(cn) * 8 : 0;
+  const size_t dbe_bytes = db ? static_cast<size_t>(bn) * 4 : 0;
+  const size_t bytes = records + db_bytes + dc_bytes + dce_bytes + dbe_bytes;
+  // Where pairs pay, per pass.  A step on pairs saves 20 us of few rays' FP64
+  // chain, 1.6 ns a ray of many rays'.  Against that stand the records: their
+  // launch and allocation, 45 us of host and device time for a forward or
+  // adjoint pass and 19 for a tangent one (one pass), 40 ps a cell to fill them,
+  // and, beyond what the pool keeps, mapping memory.  Adjoint (both passes) and
+  // tangent, FP64 -> pairs, us: 217 rays on 200^2 nodes, 1 step 422 / 56 -> 469
+  // / 58 (not taken), 5 steps 548 / 180 -> 468 / 100, 100 steps 6,977 / 3,117 ->
+  // 3,094 / 1,082; on 1,024^2, 10 steps 834 / 338 -> 931 / 468 (not taken), 20
+  // steps 1,508 / 650 -> 1,082 / 489; 32,768 rays there, 5 steps 857 / 361 ->
+  // 852 / 435 (not taken), 10 steps 1,565 / 696 -> 942 / 420.  Grids of up to
+  // 4,096 cells are on pairs at any length: such a call is the host's time, and
+  // the FP64 form's exp(-2 kh) = 1 - (1 - exp(-2 kh)) has few digits from kh = 15
+  // on.  Up to 2^24 cells, 4.9 GB of records: what a call may take beside its
+  // own buffers.
+  if (k.n == 0 || k.steps == 0 || cells > (1ll << 24) || k.bnx > (1 << 20) ||
+      k.bny > (1 << 20) || k.cnx > (1 << 20) || k.cny > (1 << 20))
     return false;
+  const double per_step = 1.6 * static_cast<double>(k.n);
+  const double saved = static_cast<double>(k.steps) * (per_step > 20e3 ? per_step : 20e3);
+  const double fixed = form == DIFF_TANGENT || cells <= 4096 ? 19e3 : 45e3;
+  const double cost = fixed + (bytes <= kKeptBytes ? 0.04 * static_cast<double>(cells)
+                                                   : 120e3 + 0.19 * static_cast<double>(cells));
+  if (cost > saved) return false;
   if (!in_range(k.dt) || !in_range(k.b_inv_dx) || !in_range(k.b_inv_dy) ||
       !in_range(k.c_inv_dx) || !in_range(k.c_inv_dy))
     return false;
@@ -1305,14 +1340,6 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   // the caller's graph).
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   char *mem = nullptr;
-  const bool db = form == DIFF_TANGENT && k.d_depth;
-  const bool dc = form == DIFF_TANGENT && (k.d_u || k.d_v);
-  const size_t records = static_cast<size_t>(bn) * 64 + static_cast<size_t>(cn) * 128;
-  const size_t db_bytes = db ? static_cast<size_t>(bn) * 32 : 0;
-  const size_t dc_bytes = dc ? static_cast<size_t>(cn) * 64 : 0;
-  const size_t dce_bytes = dc ? static_cast<size_t>(cn) * 8 : 0;
-  const size_t dbe_bytes = db ? static_cast<size_t>(bn) * 4 : 0;
-  const size_t bytes = records + db_bytes + dc_bytes + dce_bytes + dbe_bytes;
   cudaMemPool_t pool = nullptr;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
       !(pool = record_pool()) ||
