@@ -32,6 +32,12 @@
 // flush the same cell.  The per-cell accumulation runs in the working
 // precision; only the accumulation onto the node arrays is FP64.
 //
+// The recomputed states need not be the forward's to the last bit (the forward
+// may have run on pairs and this pass not, or the other way round), so a stage
+// beside a grid's edge can have no derivative here.  The ray's walk backward
+// ends there: no cell of that stage is read or added to, and the gradient
+// returned is that of the state it had come to.
+//
 // In FP64 all three run on float pairs where diff_split.cu covers the call; the
 // kernels here in double serve the rest (few ray-steps for the grid, a stream
 // under capture, grids beyond its limits).
@@ -159,7 +165,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 1) diff_adjoint_kerne
         if (st == 3 && s + 1 == last) break;  // the last step's end is not needed
         Point<T> P;
         T k[4];
-        eval(A, Y, P, k, N);
+        if (!eval(A, Y, P, k, N)) goto done;
         const T wt = st == 0 || st == 3 ? T(1) : T(2), f = st == 2 ? h : half;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 1) diff_adjoint_kerne
 #pragma unroll
           for (int q = 0; q < 4; ++q) Yn[q] = ahead[q * A.n];
         }
-        eval(A, Y, P, kd, N);
+        if (!eval(A, Y, P, kd, N)) goto done;
         const T c = st == 3 || st == 0 ? sixth : third, f = st == 2 ? h : half;
         if (st == 3) {
 #pragma unroll
@@ -213,6 +219,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 1) diff_adjoint_kerne
       for (int q = 0; q < 4; ++q) lam[q] = lam[q] + r[q] + r2[q] + r3[q] + r4[q];
     }
   }
+done:
   flush_bathy(A, acc);
   flush_current(A, acc);
 #pragma unroll

@@ -694,8 +694,9 @@ __device__ __noinline__ bool anchor_at(const SplitArgs &S, const double *yin, MA
 }
 
 // A step backward in FP64 (diff.cu), its stage states recomputed from y; the
-// node gradients go straight to the arrays.
-__device__ __noinline__ void fp64_reverse(const DiffArgs<double> &A, const double *y0,
+// node gradients go straight to the arrays.  False (nothing added) where a
+// stage has no derivative.
+__device__ __noinline__ bool fp64_reverse(const DiffArgs<double> &A, const double *y0,
                                           double *lam_io) {
   Point<double> P;
   double Y[4][4], kd[4], w[4], r[4], lam[4], sum[4];
@@ -703,15 +704,16 @@ __device__ __noinline__ void fp64_reverse(const DiffArgs<double> &A, const doubl
 #pragma unroll
   for (int q = 0; q < 4; ++q) { Y[0][q] = y0[q]; lam[q] = lam_io[q]; sum[q] = 0.0; }
   for (int st = 0; st < 3; ++st) {
-    eval(A, Y[st], P, kd);
+    if (!eval(A, Y[st], P, kd)) return false;
     for (int q = 0; q < 4; ++q) Y[st + 1][q] = y0[q] + kd[q] * (st == 2 ? h : half);
   }
+  if (!eval(A, Y[3], P, kd)) return false;
   NodeAcc<double> acc;
   acc.bkey = acc.ckey = -1;
 #pragma unroll
   for (int q = 0; q < 4; ++q) acc.d[q] = acc.u[q] = acc.v[q] = r[q] = 0.0;
   for (int st = 3; st >= 0; --st) {
-    eval(A, Y[st], P, kd);
+    if (st < 3) eval(A, Y[st], P, kd);
     const double c = (st == 0 || st == 3) ? h / 6.0 : h / 3.0;
     const double f = st == 3 ? 0.0 : st == 2 ? h : half;
     for (int q = 0; q < 4; ++q) w[q] = lam[q] * c + f * r[q];
@@ -721,6 +723,7 @@ __device__ __noinline__ void fp64_reverse(const DiffArgs<double> &A, const doubl
   flush_bathy(A, acc);
   flush_current(A, acc);
   for (int q = 0; q < 4; ++q) lam_io[q] = lam[q] + sum[q];
+  return true;
 }
 
 template <bool SAME>
@@ -773,7 +776,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4)
         pairs[row + 4 * A.n] = make_float2(NAN, NAN);
 #pragma unroll
         for (int q = 0; q < 4; ++q) yn[q] = y[q];
-        (void)fp64_rk4(A, yn);
+        if (!fp64_rk4(A, yn)) goto done;  // (diff.cu)
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) y[q] = yn[q];
@@ -803,7 +806,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4)
         double yv[4] = {y[0], y[1], y[2], y[3]}, lv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) lv[q] = lam[q] * acc.unit();
-        fp64_reverse(A, yv, lv);
+        if (!fp64_reverse(A, yv, lv)) goto done;
 #pragma unroll
         for (int q = 0; q < 4; ++q) lam[q] = lv[q] * acc.per_unit();
         anchored = false;
@@ -872,6 +875,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4)
       anchored = true;
     }
   }
+done:
   flush_bathy(S, acc);
   flush_current(S, acc);
 #pragma unroll
