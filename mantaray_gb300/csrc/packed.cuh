@@ -8,7 +8,7 @@
 // -fmad and the rounding modifiers say (measured: every one of 20,000 random
 // vadd(c, vmul(a, b)) equals fma(a, b, c)), so code that must not be
 // contracted never feeds a vmul into a vadd or vsub, unless the product is
-// exact.
+// exact: vmul_rn takes its place.
 #pragma once
 
 #include "bits.h"
@@ -55,6 +55,14 @@ MR_HD V vmul(V a, V b) { return V{a.x * b.x, a.y * b.y}; }
 MR_HD V vfma(V a, V b, V c) { return V{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
 #endif
 MR_HD V both(float a) { return V{a, a}; }
+// a b as two scalar products, which nothing contracts.
+MR_HD V vmul_rn(V a, V b) {
+#if defined(__CUDA_ARCH__)
+  return V{__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)};
+#else
+  return V{a.x * b.x, a.y * b.y};
+#endif
+}
 #if defined(__CUDACC__)
 // a + b rounded toward minus infinity.
 __device__ __forceinline__ V vadd_down(V a, V b) {
