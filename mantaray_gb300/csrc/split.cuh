@@ -39,6 +39,14 @@
 #include "packed.cuh"
 
 namespace mr {
+// The two forms of the pairs' products have names of their own, so that units
+// of both can be linked.
+#ifdef MR_SPLIT_LOW_PRODUCT
+inline namespace pairs_low_product {
+#else
+inline namespace pairs {
+#endif
+using ::mr::both;
 
 // Functions that read the tables: device code where there is a device.
 #if defined(__CUDACC__)
@@ -418,4 +426,5 @@ MR_SPLIT void split_rhs(const Sample &s, const Wave &wv, V2 *d, V2 *dk, double k
   *dk = sub(*dk, t);
 }
 
+}  // inline namespace
 }  // namespace mr
