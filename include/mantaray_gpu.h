@@ -89,7 +89,13 @@ typedef struct mr_current mr_current;
  * of depth_len values read with flat index nx*j + i (:465-471).  depth_len
  * may differ from nx*ny exactly as in the reference (lookups past the end
  * become IndexOutOfBounds, i.e. NaN).  nx, ny >= 2 (the reference panics on
- * a one-point axis at its first lookup). */
+ * a one-point axis at its first lookup).
+ *
+ * A handle holds 20 bytes a node on the device, and 32 more for the per-cell
+ * records that traces with MR_MATH_IDENTITY read, where these take at most an
+ * eighth of the device's free memory (or 32 MiB).  Without them such traces
+ * run the general kernel: the same bars, other low bits, 4 to 5 times the
+ * time. */
 int mr_bathymetry_grid(size_t nx, size_t ny, const float *x, const float *y,
                        const double *depth, size_t depth_len,
                        mr_bathymetry **out);
@@ -117,7 +123,8 @@ void mr_bathymetry_destroy(mr_bathymetry *b);
 
 /* Gridded current (replaces CartesianCurrent, src/current/
  * cartesian_current.rs:18-27 and :58-213): f64 axes and u, v with flat index
- * nx*j + i (:421-427).  nx, ny >= 2. */
+ * nx*j + i (:421-427).  nx, ny >= 2.  56 bytes a node on the device and 80 more
+ * for the records, as above. */
 int mr_current_grid(size_t nx, size_t ny, const double *x, const double *y,
                     const double *u, size_t u_len, const double *v,
                     size_t v_len, mr_current **out);

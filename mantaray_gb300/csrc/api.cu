@@ -219,26 +219,64 @@ bool split_axis_uniform(const std::vector<mr::AxisCell> &c, float a0, float sp) 
   return true;
 }
 
-// Uploads the axis cells and builds the records; without memory for them the
-// handle works as before (the general kernels).
+// SplitAxes' affine: every value is fma(i, sp, a[0]).
+bool split_axis_affine(const float *a, size_t n, float sp) {
+  for (size_t i = 0; i < n; ++i)
+    if (a[i] != fmaf(static_cast<float>(i), sp, a[0])) return false;
+  return true;
+}
+
+mr::SplitAxes split_axes(const float *x, const float *y, size_t nx, size_t ny, float spx,
+                         float spy) {
+  mr::SplitAxes s;
+  s.x.assign(x, x + nx);
+  s.y.assign(y, y + ny);
+  s.sp_x = spx;
+  s.sp_y = spy;
+  s.affine = split_axis_affine(x, nx, spx) && split_axis_affine(y, ny, spy);
+  return s;
+}
+
+// Whether two fields' axes are equal as f32: from their parameters where both
+// are affine (a call compares them each time), else value by value.
+bool same_split_axes(const mr::SplitAxes &a, const mr::SplitAxes &b) {
+  if (a.x.empty() || a.x.size() != b.x.size() || a.y.size() != b.y.size()) return false;
+  if (a.affine && b.affine && a.sp_x == b.sp_x && a.sp_y == b.sp_y)
+    return a.x[0] == b.x[0] && a.y[0] == b.y[0];
+  return a.x == b.x && a.y == b.y;
+}
+
+// Uploads the axis cells and builds the records, if split_records_fit; without
+// memory for them the handle works as before (the general kernels).
 template <typename Handle, typename Launch>
 cudaError_t make_split(Handle *h, const float *x, const float *y, size_t nx, size_t ny,
                        const std::vector<float> &fx, const std::vector<float> &fy,
                        bool inclusive, float spx, float spy, size_t record, Launch launch) {
-  const auto xc = split_axis_cells(x, nx, fx, inclusive);
-  const auto yc = split_axis_cells(y, ny, fy, inclusive);
-  void *rec = nullptr;
-  if (cudaMalloc(&rec, nx * ny * record) != cudaSuccess) {
+  const size_t bytes = nx * ny * record;
+  size_t free_bytes = 0, total = 0;
+  if (bytes > mr::kSplitSmallBytes && cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
     (void)cudaGetLastError();
     return cudaSuccess;
   }
-  h->mem.push_back(rec);
+  if (!mr::split_records_fit(bytes, free_bytes)) return cudaSuccess;
+  const auto xc = split_axis_cells(x, nx, fx, inclusive);
+  const auto yc = split_axis_cells(y, ny, fy, inclusive);
+  std::vector<void *> mem;
+  void *rec = nullptr;
   mr::SplitGrid g{};
-  cudaError_t e = upload(xc.data(), xc.size(), &h->mem, &g.xc);
-  if (e == cudaSuccess) e = upload(yc.data(), yc.size(), &h->mem, &g.yc);
+  cudaError_t e = cudaMalloc(&rec, bytes);
+  if (e == cudaSuccess) mem.push_back(rec);
+  if (e == cudaSuccess) e = upload(xc.data(), xc.size(), &mem, &g.xc);
+  if (e == cudaSuccess) e = upload(yc.data(), yc.size(), &mem, &g.yc);
   if (e == cudaSuccess) e = launch(h->dev, rec, cudaStreamPerThread);
   if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) {
+    free_mem(mem);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    return cudaSuccess;
+  }
+  h->mem.insert(h->mem.end(), mem.begin(), mem.end());
   g.rec = rec;
   g.nx = static_cast<int>(nx);
   g.ny = static_cast<int>(ny);
@@ -251,8 +289,7 @@ cudaError_t make_split(Handle *h, const float *x, const float *y, size_t nx, siz
   g.uniform_x = split_axis_uniform(xc, x[0], spx);
   g.uniform_y = split_axis_uniform(yc, y[0], spy);
   h->dev.split = g;
-  h->x32.assign(x, x + nx);
-  h->y32.assign(y, y + ny);
+  h->axes = split_axes(x, y, nx, ny, spx, spy);
   return cudaSuccess;
 }
 
@@ -473,7 +510,7 @@ int launch(const mr_bathymetry *b, const mr_current *c, size_t n, const double *
   a.traj = traj;
   a.n_rows = n_rows;
   a.status = status;
-  const bool same_axes = !b->x32.empty() && b->x32 == c->x32 && b->y32 == c->y32;
+  const bool same_axes = same_split_axes(b->axes, c->axes);
   cudaError_t e = mr::launch_rk4_f64(b->dev, c->dev, a, options & MR_STOP_FRESH,
                                      (options & MR_MATH_LIBM) == 0, same_axes, stream);
   if (e != cudaSuccess) return cuda_fail(e, "rk4_f64 launch");

@@ -8,12 +8,32 @@
 
 #include "fields.h"
 
+namespace mr {
+
+// A gridded field's axes as f32, on the host, where it has records (SplitGrid).
+struct SplitAxes {
+  std::vector<float> x, y;
+  float sp_x = 0.0f, sp_y = 0.0f;
+  bool affine = false;
+};
+
+// Records are built with the handle (the traces themselves allocate nothing)
+// and stay with it, so they may take an eighth of the free memory at most: what
+// a program allocates after its handles, such as a batch's cells, has room as
+// before.  Up to kSplitSmallBytes is not looked at.
+constexpr size_t kSplitSmallBytes = size_t(32) << 20;
+inline bool split_records_fit(size_t bytes, size_t free_bytes) {
+  return bytes <= kSplitSmallBytes || bytes <= free_bytes / 8;
+}
+
+}  // namespace mr
+
 struct mr_bathymetry {
   mr::BathyDev dev{};
   int device = 0;
   bool one_point_axis = false;  // the reference panics on its first lookup
   std::vector<void *> mem;      // device allocations owned by the handle
-  std::vector<float> x32, y32;  // host copies of the axes as f32 (grids)
+  mr::SplitAxes axes;
 };
 
 struct mr_current {
@@ -21,7 +41,7 @@ struct mr_current {
   int device = 0;
   bool one_point_axis = false;
   std::vector<void *> mem;
-  std::vector<float> x32, y32;  // host copies of the axes as f32 (grids)
+  mr::SplitAxes axes;
 };
 
 namespace mr {
