@@ -36,7 +36,7 @@ struct PackedGrid {
   float cu, cv;          // constant current
 };
 
-// Axes longer than this take the integrator's wide build (k2.cuh, locate).
+// Axes longer than this take the integrator's wide builds (k2.cuh, locate).
 constexpr int kNarrowAxis = 1 << 22;
 
 struct ScenarioDev {

@@ -49,7 +49,7 @@ struct mr_batch {
   bool has_tmaps = false;
 };
 
-// 1 when an axis of some scenario needs the integrator's wide build.
+// 1 when an axis of some scenario needs the integrator's wide builds.
 inline int wide_axes(const mr_batch *b) {
   for (const mr::ScenarioDev &s : b->host_scen)
     for (const mr::PackedGrid *g : {&s.bathy, &s.current})
@@ -81,9 +81,10 @@ inline int same_geometry(const mr_batch *b) {
 
 // The batched kernel's mode for a batch (k2.cuh).
 inline int batch_mode(const mr_batch *b) {
-  if (wide_axes(b)) return 4;
-  if (b->n_scenarios == 1) return all_same_grid(b) ? 2 : 1;
-  return same_geometry(b) ? 5 : all_same_grid(b) ? 3 : 0;
+  const int wide = wide_axes(b) ? 8 : 0;
+  if (b->n_scenarios == 1) return wide + (all_same_grid(b) ? 2 : 1);
+  if (!wide && same_geometry(b)) return 5;
+  return wide + (all_same_grid(b) ? 3 : 0);
 }
 
 struct mr_batch_config;

@@ -108,7 +108,7 @@ extern "C" int mr_batch_trace_device_static(
   // and never read the table, so one scenario needs no copy.
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : cudaStreamPerThread;
   cudaError_t e = cudaSuccess;
-  if (a.mode != 1 && a.mode != 2)  // the table builds
+  if ((a.mode & 7) != 1 && (a.mode & 7) != 2)  // the table builds
     e = cudaMemcpyAsync(table, b->scen, static_cast<size_t>(b->n_scenarios) * sizeof(mr::ScenarioDev),
                         cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);

@@ -2,10 +2,11 @@
 // two translation units that instantiate its kernels: rk4_f32.cu (the
 // scenario-table builds: MODE 0; MODE 3 when every scenario's current is
 // gridded on its bathymetry's grid, MODE 5 when besides every scenario has the
-// first one's axes; MODE 4 for very long axes) and rk4_f32_one.cu (the single-scenario
-// builds, compiled with FP32 subnormals flushed: MODE 1, and MODE 2 when the
-// current is gridded on the bathymetry's grid).  The design notes are at the
-// top of rk4_f32.cu.
+// first one's axes) and rk4_f32_one.cu (the single-scenario builds, compiled
+// with FP32 subnormals flushed: MODE 1, and MODE 2 when the current is gridded
+// on the bathymetry's grid).  Modes 8 to 11 are 0 to 3 for very long axes
+// (rk4_f32_wide.cu for 9 and 10).  The design notes are at the top of
+// rk4_f32.cu.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -23,6 +24,9 @@ namespace {
 
 constexpr int kCappedRegs = 64;  // of the capped builds (below)
 constexpr int kMiddleRegs = 72;
+// A mode without the axes' length, and whether it is for very long ones.
+__host__ __device__ constexpr int base_mode(int mode) { return mode & 7; }
+__host__ __device__ constexpr bool wide_mode(int mode) { return mode >= 8; }
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kGf = 9.8f;
 
@@ -227,14 +231,14 @@ __device__ __forceinline__ void ray_equations(float h, V uv, V du, V dv, V grad,
 
 // A lane's scenario: from the kernel's parameters in the single-scenario
 // builds (MODE 1, 2) and, for all but its records, where every scenario has
-// the same geometry (MODE 5); else from the device table (MODE 0, 3, 4).
+// the same geometry (MODE 5); else from the device table (MODE 0, 3).
 template <int MODE>
 __device__ __forceinline__ const ScenarioDev &scenario(const BatchArgs &a, int s) {
-  return (MODE == 1 || MODE == 2 || MODE == 5) ? a.scen0 : a.scen[s];
+  return (base_mode(MODE) == 1 || base_mode(MODE) == 2 || MODE == 5) ? a.scen0 : a.scen[s];
 }
 template <int MODE>
 __device__ __forceinline__ const ScenarioDev &cells_of(const BatchArgs &a, int s) {
-  return (MODE == 1 || MODE == 2) ? a.scen0 : a.scen[s];
+  return (base_mode(MODE) == 1 || base_mode(MODE) == 2) ? a.scen0 : a.scen[s];
 }
 
 // The records of bathymetry cell cb, unless the lane holds them.
@@ -511,9 +515,9 @@ __device__ __forceinline__ int rhs_f32(const ScenarioDev &s, const ScenarioDev &
   CellCache &C = L.cache;
   int cb, ix, iy;
   V f;
-  bool inside = locate<MODE == 4>(s.bathy, L.pb, p, &cb, &f, &ix, &iy);
+  bool inside = locate<wide_mode(MODE)>(s.bathy, L.pb, p, &cb, &f, &ix, &iy);
   V uv, du, dv;
-  if (MODE == 2 || MODE == 3 || MODE == 5) {
+  if (base_mode(MODE) == 2 || base_mode(MODE) == 3 || MODE == 5) {
     if (STAGE == 1)
       load_same_grid_cell_tile(s, C, W, inside ? cb : C.bkey, ix, iy);
     else if (STAGE == 2)
@@ -528,7 +532,7 @@ __device__ __forceinline__ int rhs_f32(const ScenarioDev &s, const ScenarioDev &
     if (s.current.kind == 0) {
       int cc = cb;
       V g = f;  // the same cell when the grids coincide (same origin, same arithmetic)
-      if (!s.same_grid) inside &= locate<MODE == 4>(s.current, L.pc, p, &cc, &g);
+      if (!s.same_grid) inside &= locate<wide_mode(MODE)>(s.current, L.pc, p, &cc, &g);
       load_current_cell(s, C, inside ? cc : C.ckey);
       uv = bilin2(C.c0, C.c1, g);
       du = V{C.c2.x, C.c2.y};
@@ -604,7 +608,7 @@ __device__ __forceinline__ int32_t save_period(const BatchArgs &a) {
 template <int MODE>
 __device__ __forceinline__ void start(const BatchArgs &a, RayLane &L, int64_t r) {
   L.ray = r;
-  L.scen = ((MODE == 0 || MODE >= 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
+  L.scen = (base_mode(MODE) != 1 && base_mode(MODE) != 2 && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
                                                          : 0;
   if (L.scen >= a.n_scenarios) L.scen = 0;
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
@@ -636,7 +640,7 @@ __device__ __forceinline__ void start(const BatchArgs &a, RayLane &L, int64_t r)
 template <int MODE>
 __device__ __forceinline__ void resume(const BatchArgs &a, RayLane &L, int64_t r) {
   L.ray = r;
-  L.scen = ((MODE == 0 || MODE >= 3) && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
+  L.scen = (base_mode(MODE) != 1 && base_mode(MODE) != 2 && a.ray_scenario) ? static_cast<int>(a.ray_scenario[r])
                                                          : 0;
   if (L.scen >= a.n_scenarios) L.scen = 0;
   const ScenarioDev &s = scenario<MODE>(a, L.scen);
@@ -907,11 +911,11 @@ __device__ __forceinline__ void k2_body(const BatchArgs &a) {
 // table; 1 (one scenario) takes the scenario's fields from the kernel's
 // parameters (operands of the instructions instead of loads at every
 // lookup); 2 is mode 1 and 3 is mode 0 with the current gridded on the
-// bathymetry's grid (every scenario's, for 3).  Mode 4 is mode 0 for axes of
-// more than 2^22 points (locate, WIDE), in the uncapped builds only.  Mode 5
-// is mode 3 where every scenario has the first one's axes: the geometry is in
-// the kernel's parameters and only a new cell's records go through the table
-// (mode 3 reads ten values of it in each lookup).
+// bathymetry's grid (every scenario's, for 3).  Mode 5 is mode 3 where every
+// scenario has the first one's axes: the geometry is in the kernel's
+// parameters and only a new cell's records go through the table (mode 3 reads
+// ten values of it in each lookup).  Modes 8 to 11 are 0 to 3 for axes of more
+// than 2^22 points (locate, WIDE), with the 72-register builds for capped.
 template <int MODE>
 __global__ void __launch_bounds__(256) rk4_f32_kernel_1(BatchArgs a) { k2_body<1, MODE, 0>(a); }
 template <int MODE>

@@ -55,6 +55,9 @@ size_t rk4_f32_tile_smem(int block);
 // build (3 and 4: same grid only, else null), 5 and 6 the sweep form of 0
 // and 1, 7 and 8 the middle build (kMiddleRegs) and its sweep form.
 const void *rk4_f32_one_function(int build, int same_grid);
+// The same for very long axes (rk4_f32_wide.cu): no staged builds, 72
+// registers in place of kCappedRegs.
+const void *rk4_f32_wide_function(int build, int same_grid);
 cudaError_t launch_fill_nan(float *p, int64_t count, cudaStream_t stream);
 
 // Spatial ordering of a batched call's rays (K6): sorts by key in `passes`

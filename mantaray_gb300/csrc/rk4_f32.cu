@@ -175,10 +175,22 @@ static const void *table_build(int k) {
   return builds[k];
 }
 
+// The same for a wide table mode, whose capped builds are the middle ones.
+template <int MODE>
+static const void *wide_table_build(int k) {
+  static const void *builds[6] = {reinterpret_cast<const void *>(&rk4_f32_kernel_1<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1m<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_2<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1s<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1m<MODE>),
+                                  reinterpret_cast<const void *>(&rk4_f32_kernel_1ms<MODE>)};
+  return builds[k];
+}
+
 // Resident blocks per SM of each mode's uncapped [0] and middle [1] one-ray
 // builds (plain and sweep form) by block size (multiples of 32 up to 256),
 // queried once; 0: not yet known.
-static std::atomic<int> g_resident[2][2][6][9];
+static std::atomic<int> g_resident[2][2][12][9];
 
 static int resident_blocks(const void *fn, int middle, int sweep, int mode, int block) {
   const int slot = (block >= 32 && block <= 256 && block % 32 == 0) ? block / 32 : 0;
@@ -198,9 +210,7 @@ size_t rk4_f32_tile_smem(int block) {
 
 const void *rk4_f32_function(int64_t n, int rays_per_lane, int block, int blocks_per_sm, int mode,
                              int staging, int sweep) {
-  if (mode == 4)  // results do not depend on the shape or the staging
-    return sweep ? reinterpret_cast<const void *>(&rk4_f32_kernel_1s<4>)
-                 : reinterpret_cast<const void *>(&rk4_f32_kernel_1<4>);
+  if (mode >= 8) staging = 0;  // not built for very long axes; the same results
   if (sweep && (staging != 0 || rays_per_lane != 1)) return nullptr;
   if (staging == 1) return (mode == 2 && rays_per_lane == 1) ? rk4_f32_one_function(3, 1) : nullptr;
   if (staging == 2) {
@@ -217,10 +227,13 @@ const void *rk4_f32_function(int64_t n, int rays_per_lane, int block, int blocks
   const int sw = sweep ? 1 : 0;
   const void *fn[4];
   for (int k = 0; k < 4; ++k)
-    fn[k] = mode == 1 || mode == 2 ? rk4_f32_one_function(kOneBuild[sw][k], mode == 2)
-             : mode == 5            ? table_build<5>(kTableBuild[sw][k])
-             : mode == 3            ? table_build<3>(kTableBuild[sw][k])
-                                    : table_build<0>(kTableBuild[sw][k]);
+    fn[k] = mode == 1 || mode == 2  ? rk4_f32_one_function(kOneBuild[sw][k], mode == 2)
+            : mode == 9 || mode == 10 ? rk4_f32_wide_function(kOneBuild[sw][k], mode == 10)
+            : mode == 5               ? table_build<5>(kTableBuild[sw][k])
+            : mode == 3               ? table_build<3>(kTableBuild[sw][k])
+            : mode == 11              ? wide_table_build<11>(kTableBuild[sw][k])
+            : mode == 8               ? wide_table_build<8>(kTableBuild[sw][k])
+                                      : table_build<0>(kTableBuild[sw][k]);
   if (rays_per_lane == 2) return fn[2];
   const int free_blocks = resident_blocks(fn[0], 0, sw, mode, block);
   if (free_blocks == 0 || free_blocks >= blocks_per_sm) return fn[0];
@@ -262,7 +275,7 @@ cudaError_t launch_rk4_f32(const BatchArgs &a, int block, int blocks_per_sm, int
   const void *fn = rk4_f32_function(a.n, rays_per_lane, block, blocks_per_sm, a.mode, a.staging,
                                     a.sweep_steps > 0);
   if (!fn) return cudaErrorInvalidValue;
-  const size_t smem = a.mode == 4 ? 0
+  const size_t smem = a.mode >= 8 ? 0
                       : a.staging == 1 ? rk4_f32_tile_smem(block)
                       : a.staging == 2 ? static_cast<size_t>(block) * 80 : 0;
   return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, stream);

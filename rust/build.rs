@@ -20,6 +20,7 @@ const UNITS: &[(&str, &[&str])] = &[
     ("diag.cu", &[]),
     ("rk4_f32.cu", &["-fmad=false"]),
     ("rk4_f32_one.cu", &["-fmad=false", "-ftz=true"]),
+    ("rk4_f32_wide.cu", &["-fmad=false", "-ftz=true"]),
     ("batch_api.cu", &[]),
     ("batch_static.cu", &[]),
     ("diff.cu", &[]),
