@@ -136,11 +136,15 @@ def tangent(x0, y0, kx0, ky0, depth, u, v, bgrid, cgrid, dt, steps, dstate0=None
     end = torch.empty((4, n), dtype=x0.dtype, device=x0.device)
     d_end = torch.empty((4, n), dtype=x0.dtype, device=x0.device)
     status = torch.empty(n, dtype=torch.uint8, device=x0.device)
-    ptr = (lambda t: t.contiguous().data_ptr() if t is not None else None)
+    # contiguous copies live until the launch is queued (one freed before could
+    # be the next one's memory)
+    dstate0, *fields = [None if t is None else t.contiguous() for t in (dstate0, d_depth, d_u, d_v)]
+    x0, y0, kx0, ky0, depth, u, v = (t.contiguous() for t in (x0, y0, kx0, ky0, depth, u, v))
+    ptr = (lambda t: t.data_ptr() if t is not None else None)
     N.check(N.load().mr_diff_tangent(
         p, ctypes.byref(bgrid), depth.data_ptr(), ctypes.byref(cgrid), u.data_ptr(), v.data_ptr(),
         n, x0.data_ptr(), y0.data_ptr(), kx0.data_ptr(), ky0.data_ptr(),
-        dstate0.contiguous().data_ptr(), ptr(d_depth), ptr(d_u), ptr(d_v), float(dt), int(steps),
+        dstate0.data_ptr(), *[ptr(t) for t in fields], float(dt), int(steps),
         end.data_ptr(), d_end.data_ptr(), status.data_ptr(), _stream(x0)))
     return end, d_end, status
 
