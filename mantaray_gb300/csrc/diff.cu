@@ -39,8 +39,8 @@
 // returned is that of the state it had come to.
 //
 // In FP64 all three run on float pairs where diff_split.cu covers the call; the
-// kernels here in double serve the rest (few ray-steps for the grid, a stream
-// under capture, grids beyond its limits).
+// kernels here in double serve the rest (few steps, where the records cost more
+// than they save, a stream under capture, grids beyond its limits).
 
 #include <cuda_runtime.h>
 #include <math.h>

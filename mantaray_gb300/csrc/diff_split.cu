@@ -19,15 +19,15 @@
 //                  gradients' error after 300 steps is 1.7 times FP64's).
 //
 // 32,768 rays x 300 steps on 512 x 512 nodes, forward and adjoint: 44.0 ms in
-// FP64, 14.2 ms here (13.6 with the wavenumbers' derivative in pairs alone,
+// FP64, 14.1 ms here (0.6 less with the wavenumbers' derivative in pairs alone,
 // whose error under strong refraction, depths 200 times apart in neighbouring
 // cells, was 6 times FP64's).  The recomputed forward pass and the adjoint are
 // 2,800 and 7,300 instructions a warp-step, two warps a scheduler: what is left
 // is the latency of dependent FP32 operations (2.3 of 4.6 cycles an
 // instruction), and the lanes of a warp in deep and in shallower water (22.5 of
 // 32 active).  The variant with FP64 equations in the reverse pass took 17.8 ms.
-// Tangent-linear, 8,192 rays x 500 steps: 16.2 ms in FP64, 5.8 here, one warp a
-// scheduler (5.5 with one unit for the call, which lost the tangents of every
+// Tangent-linear, 8,192 rays x 500 steps: 16.2 ms in FP64, 5.7 here, one warp a
+// scheduler (5.3 with one unit for the call, which lost the tangents of every
 // ray far below the call's largest); along a depth tangent alone 5.8 (29.6:
 // lanes parted by steps in FP64 stayed parted).
 // Error against 128-bit arithmetic over 50 to 400 steps of 1 to 4 s on 200 to
@@ -45,8 +45,9 @@
 // and, beyond a = 22, w = sqrt(g)/2 k^(-3/2), c_g,k = -w/2, the rest 0.
 //
 // Fields: one record per cell, built at the start of the call (bilinear
-// coefficients of depth, u and v in pairs and in FP64, 192 bytes), kept in
-// registers while a ray stays in the cell.  A stage's position is the step's
+// coefficients of depth, u and v in pairs and in FP64, 192 bytes; of the
+// tangent fields in pairs, 108), kept in registers while a ray stays in the
+// cell.  A stage's position is the step's
 // FP64 cell and fraction plus the displacement in pairs.
 //
 // Steps outside the pairs' domain (depth or k^2 as in split_ok, a cell
@@ -1306,7 +1307,7 @@ bool launch_diff_split(DiffForm form, const DiffCall &k, cudaStream_t stream, cu
   // 852 / 435 (not taken), 10 steps 1,565 / 696 -> 942 / 420.  Grids of up to
   // 4,096 cells are on pairs at any length: such a call is the host's time, and
   // the FP64 form's exp(-2 kh) = 1 - (1 - exp(-2 kh)) has few digits from kh = 15
-  // on.  Up to 2^24 cells, 4.9 GB of records: what a call may take beside its
+  // on.  Up to 2^24 cells, 5.0 GB of records: what a call may take beside its
   // own buffers.
   if (k.n == 0 || k.steps == 0 || cells > (1ll << 24) || k.bnx > (1 << 20) ||
       k.bny > (1 << 20) || k.cnx > (1 << 20) || k.cny > (1 << 20))

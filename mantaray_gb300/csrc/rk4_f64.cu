@@ -151,7 +151,8 @@ cudaError_t launch_rk4_f64(const BathyDev &b, const CurrentDev &c, const TraceAr
   if (a.n == 0) return cudaSuccess;
   // Blocks of 64 rays, or fewer when that leaves SMs without a block: on
   // GB300 an SM issues 2 FP64 lanes per clock, so a small call runs fastest
-  // with its rays spread over as many SMs as possible (down to 8 per block).
+  // with its rays spread over as many SMs as possible (down to 8 per block:
+  // fewer gained nothing in the FP64 form; not measured for the split form).
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
